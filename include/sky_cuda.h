@@ -256,8 +256,9 @@ typedef struct SkyDeviceOutputs {
  * candidates of these on the caller's workload and keeps the fastest.
  */
 typedef struct SkyTuning {
-    uint32_t variant;            /* resident blocks of 256 threads per SM the kernel is compiled
-                                    for: 0 = 3 (80 registers), 1 = 2 (128), 2 = 4 (64)         */
+    uint32_t variant;            /* warps per SM the kernel is compiled for: 0 = 24 (80 registers
+                                    per lane), 1 = 16 (128), 2 = 32 (64); renders of few chains
+                                    per lane always run the last                                */
     uint32_t max_blocks_per_sm;  /* 0 = occupancy limit                                          */
     uint32_t all_species;        /* 1 = the kernels evaluate all four aerosol species; 0 = only
                                     species 0 when species 1-3 carry no aerosol anywhere in the
@@ -266,9 +267,10 @@ typedef struct SkyTuning {
     float crossing_cost;         /* merged tracking grid: cost of a layer crossing relative to a
                                     null collision; <= 0 leaves the grid as it is              */
     uint32_t iteration_limit;    /* backstop of the wavefront kernel: loop iterations (one ray
-                                    per lane each) a warp may run before it stops and reports
-                                    SKY_ERR_WATCHDOG; 0 = 2^31.  A render needs about
-                                    3 x chains / (32 x resident warps) iterations per warp.    */
+                                    per lane each, or four batches of the stage queues) a warp
+                                    may run before it stops and reports SKY_ERR_WATCHDOG;
+                                    0 = 2^31.  A render needs about 3 x chains / (32 x resident
+                                    warps) iterations per warp.                              */
     uint32_t _reserved[2];
 } SkyTuning;
 

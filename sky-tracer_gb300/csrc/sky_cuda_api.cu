@@ -47,11 +47,11 @@ struct SkyScene {
     uint64_t ws_cells = 0, ws_pixels = 0;
     // wavefront-kernel job table and work counter (one job per render call)
     DevJob* jobs = nullptr;
-    uint32_t* work_counter = nullptr;
+    unsigned long long* work_counter = nullptr;
     // batch job tables: device table + pinned host staging, grown on demand
     DevJob* batch_jobs = nullptr;
     DevJob* batch_host = nullptr;
-    uint32_t* batch_counter = nullptr;
+    unsigned long long* batch_counter = nullptr;
     uint32_t batch_capacity = 0;
     SkyTuning tuning{};
     // merged tracking grid in its own allocation (rebuilt by set_tuning)
@@ -222,6 +222,7 @@ DevLaunch make_launch(const SkyScene* s, const SkyRenderConfig* c) {
     L.observer_altitude = c->observer_altitude_km;
     L.inv_width = 1.0f / float(c->width);
     L.inv_height = 1.0f / float(c->height);
+    L.spp_reciprocal = ~uint64_t(0) / c->spp;
     const float rg = s->dev.ground_radius;
     const float oy = rg + std::max(c->observer_altitude_km, 0.0f);
     const float view_height = std::sqrt(0.0f * 0.0f + oy * oy + 0.0f * 0.0f);
@@ -251,19 +252,23 @@ DevLaunch make_launch(const SkyScene* s, const SkyRenderConfig* c) {
 constexpr uint64_t kMaxLaunchCells = 0xF0000000ull;
 
 // Place a job in the launch's cell space after the cells already placed.
-int place_job(DevJob& job, uint64_t pixels, uint32_t bands, uint64_t& cells_so_far, uint32_t& max_cells) {
+int place_job(DevJob& job, uint64_t pixels, uint32_t bands, uint64_t& cells_so_far, uint32_t& max_cells,
+              uint64_t& chains_so_far) {
     const uint64_t cells = pixels * bands;
     if (cells_so_far + cells > kMaxLaunchCells)
         return set_error(SKY_ERR_INVALID_CONFIG, "a launch holds at most 4026531840 (pixel, band) cells");
     job.cell_begin = uint32_t(cells_so_far);
     job.cell_count = uint32_t(cells);
+    job.chain_begin = chains_so_far;
     cells_so_far += cells;
+    chains_so_far += cells * job.L.spp;
     max_cells = std::max(max_cells, uint32_t(cells));
     return SKY_OK;
 }
 
 WaveLaunch wave_launch(const SkyScene* s, const DevJob& first, const DevJob* dev_jobs, uint32_t n, uint64_t cells,
-                       uint32_t max_cells, uint32_t tracking, uint32_t phase_sampling, uint32_t* counter,
+                       uint32_t max_cells, uint64_t chains, uint32_t tracking, uint32_t phase_sampling,
+                       unsigned long long* counter,
                        unsigned long long* counters, uint32_t* status) {
     WaveLaunch w{};
     w.scene = first.S;
@@ -272,6 +277,7 @@ WaveLaunch wave_launch(const SkyScene* s, const DevJob& first, const DevJob* dev
     w.num_jobs = n;
     w.total_cells = uint32_t(cells);
     w.max_job_cells = max_cells;
+    w.total_chains = chains;
     w.variant = s->tuning.variant;
     w.max_blocks_per_sm = s->tuning.max_blocks_per_sm;
     w.tracking = tracking;
@@ -324,9 +330,10 @@ int launch_render(SkyScene* s, const SkyRenderConfig* c, const SkyDeviceOutputs*
     job.total_spp = total_spp;
     uint64_t cells = 0;
     uint32_t max_cells = 0;
-    int st = place_job(job, pixels, s->dev.band_count, cells, max_cells);
+    uint64_t chains = 0;
+    int st = place_job(job, pixels, s->dev.band_count, cells, max_cells, chains);
     if (st) return st;
-    const WaveLaunch w = wave_launch(s, job, s->jobs, 1, cells, max_cells, c->tracking, c->phase_sampling,
+    const WaveLaunch w = wave_launch(s, job, s->jobs, 1, cells, max_cells, chains, c->tracking, c->phase_sampling,
                                      s->work_counter, o->counters, o->status);
     if ((e = cudaMemcpyAsync(s->jobs, &job, sizeof(job), cudaMemcpyHostToDevice, stream)) != cudaSuccess)
         return cuda_fail(SKY_ERR_COPY, "job upload", e);
@@ -618,7 +625,7 @@ int sky_cuda_scene_create(const SkySceneDesc* desc, SkyScene** out_scene) {
                                      std::to_string(sp) + " has mass and optics";
     }
     if ((e = dev_malloc(&s->jobs, sizeof(DevJob))) != cudaSuccess ||
-        (e = dev_malloc(&s->work_counter, sizeof(uint32_t))) != cudaSuccess) {
+        (e = dev_malloc(&s->work_counter, sizeof(*s->work_counter))) != cudaSuccess) {
         sky_cuda_scene_destroy(s);
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "job table allocation", e);
     }
@@ -702,7 +709,7 @@ struct SkyBatchGraph {
     int device = 0;                // the scene's device, kept: the graph may outlive its scene handle
     DevJob* jobs = nullptr;        // device job table owned by the graph
     DevJob* host = nullptr;        // pinned copy the graph's memcpy node reads
-    uint32_t* counter = nullptr;
+    unsigned long long* counter = nullptr;
     uint32_t job_count = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -712,12 +719,13 @@ namespace {
 
 // Fill DevJob rows for a batch; returns the batch's cells and its largest job.
 int build_batch_jobs(SkyScene* s, const SkyBatchJob* jobs, uint32_t n, DevJob* out, uint64_t& cells,
-                     uint32_t& max_cells) {
+                     uint32_t& max_cells, uint64_t& chains) {
     if (!s || !jobs || n == 0) return set_error(SKY_ERR_INVALID_CONFIG, "scene and at least one job are required");
     if (!jobs[0].outputs.status) return set_error(SKY_ERR_INVALID_CONFIG, "jobs[0].outputs.status is required");
     if (n > 65535u) return set_error(SKY_ERR_INVALID_CONFIG, "a batch holds at most 65535 jobs");
     cells = 0;
     max_cells = 0;
+    chains = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const SkyRenderConfig* c = &jobs[i].config;
         int st = validate_config(s, c);
@@ -751,7 +759,7 @@ int build_batch_jobs(SkyScene* s, const SkyBatchJob* jobs, uint32_t n, DevJob* o
         job.rgb = s->has_xyz ? jobs[i].outputs.rgb : nullptr;
         job.accumulate = accumulate ? 1u : 0u;
         job.total_spp = accumulate ? c->sample_offset + c->spp : c->spp;
-        if ((st = place_job(job, slab_pixels(c), s->dev.band_count, cells, max_cells))) return st;
+        if ((st = place_job(job, slab_pixels(c), s->dev.band_count, cells, max_cells, chains))) return st;
     }
     return SKY_OK;
 }
@@ -769,7 +777,7 @@ int ensure_batch_capacity(SkyScene* s, uint32_t n) {
     cudaError_t e;
     if ((e = dev_malloc(&s->batch_jobs, size_t(n) * sizeof(DevJob))) != cudaSuccess ||
         (e = cudaMallocHost(&s->batch_host, size_t(n) * sizeof(DevJob))) != cudaSuccess ||
-        (e = dev_malloc(&s->batch_counter, sizeof(uint32_t))) != cudaSuccess)
+        (e = dev_malloc(&s->batch_counter, sizeof(*s->batch_counter))) != cudaSuccess)
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "batch job table allocation", e);
     s->batch_capacity = n;
     return SKY_OK;
@@ -789,12 +797,13 @@ extern "C" int sky_cuda_render_batch(const SkyScene* scene, const SkyBatchJob* j
     cudaStreamSynchronize(stream);
     uint64_t cells = 0;
     uint32_t max_cells = 0;
-    if ((st = build_batch_jobs(s, jobs, job_count, s->batch_host, cells, max_cells))) return st;
+    uint64_t chains = 0;
+    if ((st = build_batch_jobs(s, jobs, job_count, s->batch_host, cells, max_cells, chains))) return st;
     clear_stale_error();
     cudaError_t e = cudaMemcpyAsync(s->batch_jobs, s->batch_host, size_t(job_count) * sizeof(DevJob),
                                     cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return cuda_fail(SKY_ERR_COPY, "batch job table upload", e);
-    const WaveLaunch w = wave_launch(s, s->batch_host[0], s->batch_jobs, job_count, cells, max_cells,
+    const WaveLaunch w = wave_launch(s, s->batch_host[0], s->batch_jobs, job_count, cells, max_cells, chains,
                                      jobs[0].config.tracking, jobs[0].config.phase_sampling, s->batch_counter,
                                      jobs[0].outputs.counters, jobs[0].outputs.status);
     e = launch_trace_wave(w, stream);
@@ -814,15 +823,16 @@ extern "C" int sky_cuda_batch_graph_create(const SkyScene* scene, const SkyBatch
     g->job_count = job_count;
     uint64_t cells = 0;
     uint32_t max_cells = 0;
+    uint64_t chains = 0;
     cudaError_t e;
     int st = SKY_OK;
     cudaStream_t cap = nullptr;
     if ((e = cudaMallocHost(&g->host, size_t(std::max(job_count, 1u)) * sizeof(DevJob))) != cudaSuccess ||
         (e = dev_malloc(&g->jobs, size_t(std::max(job_count, 1u)) * sizeof(DevJob))) != cudaSuccess ||
-        (e = dev_malloc(&g->counter, sizeof(uint32_t))) != cudaSuccess) {
+        (e = dev_malloc(&g->counter, sizeof(*g->counter))) != cudaSuccess) {
         st = cuda_fail(SKY_ERR_OUT_OF_MEMORY, "batch graph allocation", e);
-    } else if ((st = build_batch_jobs(s, jobs, job_count, g->host, cells, max_cells)) == SKY_OK) {
-        const WaveLaunch w = wave_launch(s, g->host[0], g->jobs, job_count, cells, max_cells,
+    } else if ((st = build_batch_jobs(s, jobs, job_count, g->host, cells, max_cells, chains)) == SKY_OK) {
+        const WaveLaunch w = wave_launch(s, g->host[0], g->jobs, job_count, cells, max_cells, chains,
                                          jobs[0].config.tracking, jobs[0].config.phase_sampling, g->counter,
                                          jobs[0].outputs.counters, jobs[0].outputs.status);
         clear_stale_error();
@@ -1444,7 +1454,7 @@ namespace {
 
 struct NoAllocScratch {
     DevJob jobs[SKY_NOALLOC_MAX_JOBS];
-    uint32_t work_counter;
+    unsigned long long work_counter;
 };
 static_assert(sizeof(NoAllocScratch) <= SKY_NOALLOC_SCRATCH_BYTES, "scratch area too small");
 
@@ -1488,6 +1498,7 @@ extern "C" int sky_cuda_render_batch_noalloc(const SkyScene* scene, const SkyRen
     std::memset(&table, 0, sizeof(table));
     uint64_t cells = 0;
     uint32_t max_cells = 0;
+    uint64_t chains = 0;
     for (uint32_t i = 0; i < job_count; ++i) {
         const SkyRenderConfig* c = &job_configs[i];
         int st = validate_config(s, c);
@@ -1510,7 +1521,7 @@ extern "C" int sky_cuda_render_batch_noalloc(const SkyScene* scene, const SkyRen
         job.rgb = s->has_xyz ? outputs[i].rgb : nullptr;
         job.accumulate = accumulate ? 1u : 0u;
         job.total_spp = accumulate ? c->sample_offset + c->spp : c->spp;
-        if ((st = place_job(job, slab_pixels(c), s->dev.band_count, cells, max_cells))) return st;
+        if ((st = place_job(job, slab_pixels(c), s->dev.band_count, cells, max_cells, chains))) return st;
     }
     table.words = uint32_t(job_count * sizeof(DevJob) / 4u);
     if (cudaSetDevice(s->device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "cannot select the device");
@@ -1523,11 +1534,11 @@ extern "C" int sky_cuda_render_batch_noalloc(const SkyScene* scene, const SkyRen
     clear_stale_error();
     noalloc_install_kernel<<<1, 256, 0, stream>>>(table);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(SKY_ERR_LAUNCH, "job table install launch", e);
-    uint32_t* counter = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(scratch) +
-                                                    offsetof(NoAllocScratch, work_counter));
+    unsigned long long* counter = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) +
+                                                                        offsetof(NoAllocScratch, work_counter));
     // the launch resets the work counter itself
     const WaveLaunch w = wave_launch(s, table.jobs[0], static_cast<const DevJob*>(scratch), job_count, cells,
-                                     max_cells, job_configs[0].tracking, job_configs[0].phase_sampling, counter,
+                                     max_cells, chains, job_configs[0].tracking, job_configs[0].phase_sampling, counter,
                                      outputs[0].counters, outputs[0].status);
     e = launch_trace_wave(w, stream);
     if (e != cudaSuccess) return cuda_fail(SKY_ERR_LAUNCH, "wavefront tracing launch", e);

@@ -123,6 +123,7 @@ struct DevLaunch {
     float lut_forward[3];
     float lut_side[3];
     float inv_width, inv_height;
+    uint64_t spp_reciprocal;  // floor((2^64 - 1) / spp)
 };
 
 // One render inside a persistent launch: its scene (tables may be shared
@@ -143,6 +144,7 @@ struct DevJob {
     uint32_t total_spp;   // samples behind the sums after this launch
     uint32_t cell_begin;  // first global cell of the job
     uint32_t cell_count;  // width * height * bands
+    uint64_t chain_begin; // first chain of the job in the launch (cells times samples of the jobs before it)
 };
 
 }  // namespace sky

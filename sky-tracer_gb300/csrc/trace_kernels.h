@@ -22,10 +22,9 @@ cudaError_t launch_trace_plain(const DevScene& S, const DevLaunch& L, double* ce
                                unsigned long long* counters, uint32_t* status, bool accumulate,
                                uint32_t aerosol_species, cudaStream_t stream);
 
-// Persistent wavefront tracer (trace_wave.cu): a ray loop with per-lane chain
-// regeneration over a job table.
-constexpr uint32_t kWaveThreads = 256;
-constexpr uint32_t kWaveVariants = 3;  // resident blocks per SM: variant 0 -> 3, 1 -> 2, 2 -> 4
+// Persistent wavefront tracer (trace_wave.cu): stage queues over a pool of paths per block,
+// over a job table.
+constexpr uint32_t kWaveVariants = 3;  // warps per block (two blocks per SM): variant 0 -> 12, 1 -> 8, 2 -> 16
 
 struct WaveLaunch {
     DevScene scene;                // the first job's scene: its tables and constants are every job's
@@ -35,11 +34,12 @@ struct WaveLaunch {
     uint32_t num_jobs;             // at most 65535
     uint32_t total_cells;          // sum of the jobs' cell counts
     uint32_t max_job_cells;        // cells of the largest job
+    uint64_t total_chains;         // sum over the jobs of cells times samples
     uint32_t variant;              // kernel shape, < kWaveVariants
     uint32_t max_blocks_per_sm;    // 0 = as many as fit
     uint32_t tracking, phase_sampling;
     uint32_t aerosol_species;      // 1 or kSpecies (aerosol_species())
-    uint32_t* work_counter;        // reset by the launch itself
+    unsigned long long* work_counter;  // reset by the launch itself
     unsigned long long* counters;  // may be null
     uint32_t* status;
     uint32_t iteration_limit;      // loop iterations per warp before status bit 2 (SkyTuning.iteration_limit)
@@ -49,7 +49,11 @@ struct WaveLaunch {
 // the jobs' cell sums (zeroed first unless a job accumulates), film, XYZ,
 // XYZ variance and linear sRGB.
 cudaError_t launch_trace_wave(const WaveLaunch& w, cudaStream_t stream);
-// The tracing kernel alone, per tracking mode (trace_wave_*.cu).
+// The tracing kernels alone, per tracking mode: the ray loop of small renders
+// (trace_ray_*.cu) and the stage queues (trace_wave_*.cu).
+cudaError_t launch_ray_segment_restart(const WaveLaunch& w, cudaStream_t stream);
+cudaError_t launch_ray_residual_carry(const WaveLaunch& w, cudaStream_t stream);
+cudaError_t launch_ray_merged_layers(const WaveLaunch& w, cudaStream_t stream);
 cudaError_t launch_wave_segment_restart(const WaveLaunch& w, cudaStream_t stream);
 cudaError_t launch_wave_residual_carry(const WaveLaunch& w, cudaStream_t stream);
 cudaError_t launch_wave_merged_layers(const WaveLaunch& w, cudaStream_t stream);

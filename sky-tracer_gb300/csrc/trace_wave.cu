@@ -1,7 +1,8 @@
 // trace_wave.cu — the launch sequence of the wavefront tracer: prepare (zero
 // the sums of jobs that do not accumulate, reset the work counter), trace
-// (trace_wave.cuh, instantiated per tracking mode in trace_wave_*.cu) and
-// finalize (film, XYZ, variance, linear sRGB of every job).
+// (trace_wave.cuh, or trace_ray.cuh for small renders, instantiated per
+// tracking mode in trace_wave_*.cu and trace_ray_*.cu) and finalize (film, XYZ,
+// variance, linear sRGB of every job).
 
 #include <algorithm>
 
@@ -13,9 +14,9 @@ namespace {
 // Zero the sums of every job that does not accumulate (blockIdx.y = job) and
 // reset the work counter.
 __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restrict__ jobs,
-                                                           uint32_t* __restrict__ work_counter) {
+                                                           unsigned long long* __restrict__ work_counter) {
     const DevJob& J = jobs[blockIdx.y];
-    if (blockIdx.x == 0u && blockIdx.y == 0u && threadIdx.x == 0u) *work_counter = 0u;
+    if (blockIdx.x == 0u && blockIdx.y == 0u && threadIdx.x == 0u) *work_counter = 0ull;
     if (J.accumulate) return;
     double* sum = J.cell_sum;
     double* sq = J.cell_sumsq;
@@ -24,6 +25,25 @@ __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restr
         sum[i] = 0.0;
         if (sq) sq[i] = 0.0;
     }
+}
+
+// Whether a launch goes to the ray loop (trace_ray.cuh) rather than to the stage
+// queues (trace_wave.cuh): where it has so few chains per lane of the chip
+// (1024 lanes per SM) that its longest chains decide its time.  Measured with
+// both kernels (ms, ray loop against queues):
+//   merged layers      3.1 M chains 0.63 / 0.68, 5.2 M 0.97 / 0.90 (one species);
+//                      4.0 M 1.46 / 1.51, 6.7 M 2.12 / 1.77 (four): 28 per lane
+//   residual carry     1.3 M 1.34 / 1.37, 2.1 M 1.94 / 1.89: 10 per lane
+//   segment restart    0.67 M 1.26 / 1.43, 1.0 M 1.64 / 1.28: 6 per lane
+cudaError_t small_render(const WaveLaunch& w, bool& small) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint64_t per_lane = w.tracking == SKY_TRACKING_SEGMENT_RESTART  ? 6u
+                              : w.tracking == SKY_TRACKING_RESIDUAL_CARRY ? 10u
+                                                                          : 28u;
+    small = w.total_chains < per_lane * 1024u * uint64_t(sms);
+    return e;
 }
 
 }  // namespace
@@ -35,10 +55,18 @@ cudaError_t launch_trace_wave(const WaveLaunch& w, cudaStream_t stream) {
     wave_prepare_kernel<<<dim3(std::max(xblocks, 1u), w.num_jobs), 256, 0, stream>>>(w.jobs, w.work_counter);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    bool small = false;
+    if ((e = small_render(w, small)) != cudaSuccess) return e;
     switch (w.tracking) {
-        case SKY_TRACKING_SEGMENT_RESTART: e = launch_wave_segment_restart(w, stream); break;
-        case SKY_TRACKING_RESIDUAL_CARRY: e = launch_wave_residual_carry(w, stream); break;
-        case SKY_TRACKING_MERGED_LAYERS: e = launch_wave_merged_layers(w, stream); break;
+        case SKY_TRACKING_SEGMENT_RESTART:
+            e = small ? launch_ray_segment_restart(w, stream) : launch_wave_segment_restart(w, stream);
+            break;
+        case SKY_TRACKING_RESIDUAL_CARRY:
+            e = small ? launch_ray_residual_carry(w, stream) : launch_wave_residual_carry(w, stream);
+            break;
+        case SKY_TRACKING_MERGED_LAYERS:
+            e = small ? launch_ray_merged_layers(w, stream) : launch_wave_merged_layers(w, stream);
+            break;
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;

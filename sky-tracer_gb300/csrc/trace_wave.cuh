@@ -1,29 +1,42 @@
-// trace_wave.cuh — the wavefront tracing kernel (a ray loop with per-lane
-// chain regeneration over a job table) and its launch shapes, included by one
-// translation unit per tracking mode (trace_wave_*.cu) so that its
-// instantiations compile in parallel.  trace_wave.cu holds the launch
-// sequence (prepare, trace, finalize).
+// trace_wave.cuh — the wavefront tracing kernel (stage queues over a pool of
+// paths) and its launch shapes, included by one translation unit per tracking
+// mode (trace_wave_*.cu) so that its instantiations compile in parallel.
+// trace_wave.cu holds the launch sequence (prepare, trace, finalize).
 //
-// The plain kernel runs every chain to completion inside one lane, so a warp
-// executes the union of 32 different paths.  Here a chain is a sequence of
-// rays: the camera / continuation ray of each vertex and the sun shadow ray
-// of each NEE sample.  Every iteration of the kernel's loop traces exactly
-// one ray per lane through the one inlined tracker (sample_real_collision /
-// delta_transmittance, sky_trace.wgsl:405-475); the event code (scattering,
-// NEE, ground, Russian roulette, sky_trace.wgsl:566-776) then runs up to the
-// lane's next ray.  A lane whose chain ends takes the next sample of its
-// warp's current (pixel, band) cell, and the warp takes a new cell from a
-// global counter when the cell's samples run out.  So the 32 lanes enter the
-// tracker together on every iteration whatever vertex or chain each is at,
-// no lane waits for the slowest chain of a cell, and nothing waits at a block
-// barrier.
+// The work of a chain falls into four stages:
+//
+//   track     a ray's next steps through the medium (sample_real_collision and
+//             delta_transmittance, sky_trace.wgsl:405-475)
+//   vertex    a primary ray that collided or reached the ground: the vertex and
+//             its next sun sample (sky_trace.wgsl:566-608, 718-749)
+//   continue  a vertex whose sun sample is decided: its NEE term, the next
+//             direction, Russian roulette (sky_trace.wgsl:691-701, 728-767)
+//   start     a chain that ended: its radiance, and the next sample's camera ray
+//
+// A block keeps its paths in shared memory and one queue of path numbers per
+// stage.  A warp takes up to 32 paths from one queue, runs that one stage on
+// them, tracks the rays that come out of it, and puts each path into the queue
+// of the stage that it needs next.  So the lanes of a warp run the same code
+// whatever pixel, chain or vertex their paths are at; nothing waits at a block
+// barrier.  A warp leaves the tracking loop when few of its rays are still
+// under way: those go to the track queue and continue in a fuller warp.
+//
+// What bounds it: instruction issue.  HBM and the tensor cores have no part in
+// it (16 B leave the chip per cell, and a path is a chain of branches).  The
+// kernel before this one kept each lane's path in registers and ran all event
+// code once per ray: 9.5 of 32 lanes active per instruction, 7.9 G warp
+// instructions and 7.42 ms for 42 M chains (128x64, 81 bands, 64 spp).  Here
+// 21.5 lanes are active, for 5.0 G instructions and 5.15 ms; what is left is
+// the rays' different lengths, the queues (about 60 instructions to take a
+// batch and 60 to put it back, for some 800 that work on it) and instruction
+// fetch (a third of the stalls: the stages are large, and a scheduler's warps
+// are in different ones).  Tracking right after the stage, instead of queueing
+// every ray for it, took 6.2 to 5.4 ms, staying with a stage 5.4 to 5.15.
 //
 // Each chain consumes its random stream in the plain kernel's order
 // (trace_path, sky_trace.wgsl:703-776), so both kernels trace the same paths.
-// A lane keeps the FP64 sums of its current cell in registers and adds them
-// to the job's cell sums when it moves to another cell; the cells' sums
-// therefore add in no fixed order (they agree with the plain kernel's to FP64
-// rounding).
+// Radiances are added to the job's cell sums by FP64 reductions in L2, in no
+// fixed order (the sums agree with the plain kernel's to FP64 rounding).
 //
 // A launch is three kernels: prepare (zero the sums of jobs that do not
 // accumulate, reset the work counter), trace, and finalize (mean film, XYZ
@@ -33,280 +46,513 @@
 
 #include <algorithm>
 
-#include "sky_device.cuh"
-#include "trace_kernels.h"
+#include "trace_common.cuh"
 
 namespace sky {
 namespace wave {
 
+// Batches of a warp that count as one iteration of SkyTuning.iteration_limit (32
+// chains take about 3.7 batches and 3 rays).
+constexpr uint64_t kBatchesPerIteration = 4;
+constexpr uint32_t kMaxIdlePolls = 1u << 30;   // polls of empty queues (>= 100 ns each) before the same
+constexpr uint32_t kMaxSlotPolls = 1u << 24;   // polls of one queue slot before the same
 
-constexpr uint32_t kFull = 0xffffffffu;
-constexpr uint32_t kNoCell = 0xffffffffu;
-// Default backstop on the loop iterations of one warp (one ray per lane
-// each; SkyTuning.iteration_limit overrides it); a render needs ~3 rays per
-// chain / lanes in flight.  Beyond it the warp sets status bit 2 and returns.
-constexpr uint32_t kMaxIterations = 1u << 31;
+// Rays still under way when a warp leaves the tracking loop and puts them back:
+// most of a warp's rays end within a few steps, a few take many times that.
+// Merged layers: 4 to 16 measured within 1 % of each other (128x64, 81 bands, 64
+// spp); the other modes, layer by layer: 8 is 6 % slower than 12, 16 the same.
+constexpr uint32_t kPark = 8, kParkLayered = 12;
 
-// What a lane does next.
-enum : uint32_t {
-    kTrace = 0u,    // a ray is set up: trace it in the next tracking step
-    kStart = 1u,    // a new chain: camera ray
-    kPrimary = 2u,  // depth checks and the boundary of the vertex's outgoing ray
-    kLights = 3u,   // the vertex's next NEE sample, else its continuation
-    kEnd = 4u,      // the chain's radiance is final
-    kIdle = 5u      // no chain
-};
 
-// Job of global cell `g`: the last job whose first cell is <= g.
-__device__ __forceinline__ uint32_t job_of(const DevJob* __restrict__ jobs, uint32_t num_jobs, uint32_t g) {
-    uint32_t lo = 0u, hi = num_jobs;
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&jobs[mid].cell_begin) <= g) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
+// Blocks per SM.  A kernel shape is the warps of a block (SkyTuning.variant).
+constexpr int kBlocksPerSm = 2;
 
-// The launch constants and the sun frame of a lane's job: kernel parameters
-// when the launch holds one job, the job table otherwise.
-template <bool kSingle>
-__device__ __forceinline__ const DevLaunch& job_launch(const DevLaunch& L0, const DevJob* jobs, uint32_t job) {
-    if constexpr (kSingle) return L0;
-    else return jobs[job].L;
-}
-template <bool kSingle>
-__device__ __forceinline__ const DevScene& job_scene(const DevScene& S0, const DevJob* jobs, uint32_t job) {
-    if constexpr (kSingle) return S0;
-    else return jobs[job].S;
-}
+enum : uint32_t { kQTrack = 0u, kQVertex = 1u, kQContinue = 2u, kQStart = 3u, kQueues = 4u, kQNone = 7u };
 
-// Bytes of shared memory that stage_medium() fills: the band-independent knot
-// profile (48 B per knot), the per-band constants (32 B per band) and aerosol
-// optics (32 B per band), the union knots and the knot finder.
-__host__ __device__ inline size_t staged_medium_bytes(uint32_t knots, uint32_t bands) {
-    return size_t(knots) * sizeof(DevProfileKnot) + size_t(bands) * sizeof(DevBand) +
-           size_t(bands) * kSpecies * sizeof(SkyAerosolOptics) + size_t(knots) * sizeof(float) +
-           size_t(kFinderCells) * sizeof(uint16_t);
-}
+// How a ray ended (Path B.y): a real collision at t, the boundary, or no ray
+// at all (the chain's radiance is final; the path has no chain yet).
+enum : uint32_t { kHit = 1u, kMiss = 2u, kOver = 3u, kFresh = 4u };
 
-// Copy the medium tables every collision and NEE evaluation reads into the
-// block's shared memory (once per block, before the loop), and return the
-// view of them.  The per-band extinction rows and the phase tables stay in
-// global memory, read through the L1 cache.
-__device__ __forceinline__ Medium stage_medium(const DevScene& S, unsigned char* smem) {
-    DevProfileKnot* profile = reinterpret_cast<DevProfileKnot*>(smem);
-    DevBand* bands = reinterpret_cast<DevBand*>(profile + S.knot_count);
-    SkyAerosolOptics* optics = reinterpret_cast<SkyAerosolOptics*>(bands + S.band_count);
-    float* knot_z = reinterpret_cast<float*>(optics + S.band_count * kSpecies);
-    uint16_t* finder = reinterpret_cast<uint16_t*>(knot_z + S.knot_count);
-    // 4-byte words throughout (every table is a multiple of 4 bytes; the finder's 512 halves are 256 words)
-    auto copy = [](void* dst, const void* src, size_t bytes) {
-        uint32_t* d = static_cast<uint32_t*>(dst);
-        const uint32_t* s = static_cast<const uint32_t*>(src);
-        for (size_t i = threadIdx.x; i < bytes / 4u; i += blockDim.x) d[i] = __ldg(s + i);
-    };
-    copy(profile, S.profile, size_t(S.knot_count) * sizeof(DevProfileKnot));
-    copy(bands, S.bands, size_t(S.band_count) * sizeof(DevBand));
-    copy(optics, S.optics, size_t(S.band_count) * kSpecies * sizeof(SkyAerosolOptics));
-    copy(knot_z, S.knot_z, size_t(S.knot_count) * sizeof(float));
-    copy(finder, S.finder, size_t(kFinderCells) * sizeof(uint16_t));
-    __syncthreads();
-    return Medium{knot_z, finder, profile, bands, optics};
-}
+enum : uint32_t { kFlagShadow = 1u << 8, kFlagGround = 1u << 9, kFlagTop = 1u << 10 };
 
-// The medium coefficients at each lane's current scattering vertex, kept in
-// shared memory (one word per thread per value, thread-minor) from the real
-// collision that made the vertex to its NEE terms and its continuation, so
-// that a vertex evaluates coefficients_at() once instead of three times
-// (-1.6 % on the production render): the Rayleigh coefficient, the kAer
-// species' scattering coefficients and the total scattering coefficient.
+// A path in shared memory: rows of 16 bytes.
+//   A  the ray's geometry: b, p, |o|^2, t_max
+//   B  the tracker's state: t, two words of its own (how the ray ended, once it
+//      has), the position in the random stream
+//   C  the stream's keys of pixel and sample; band, flags and the tracker's
+//      layer; job and the vertex's sun samples so far
+//   D  vertex (ray origin) and throughput
+//   E  direction and radiance
+//   F  depth, cell, the vertex's NEE sum, the cosine of its sun sample
+//   G  (H) the medium at the vertex: Rayleigh, total and species' scattering
+// The row count is odd, so that the 16-byte accesses of neighbouring paths
+// fall into different banks.
+enum : uint32_t { kA = 0u, kB = 1u, kC = 2u, kD = 3u, kE = 4u, kF = 5u, kG = 6u, kH = 7u };
 template <int kAer>
-struct VertexCoeffCache {
-    float* at;  // this thread's first word
-    __device__ __forceinline__ void store(const Coeffs& c) const {
-        at[0] = c.rayleigh;
-#pragma unroll
-        for (int i = 0; i < kAer; ++i) at[(1 + i) * kWaveThreads] = c.sca[i];
-        at[(1 + kAer) * kWaveThreads] = c.scattering;
-    }
-    // What the NEE term and the continuation read: rayleigh, sca[] and
-    // scattering (the species beyond kAer are 0; absorption is not kept).
-    __device__ __forceinline__ Coeffs load() const {
-        Coeffs c;
-        c.rayleigh = at[0];
-#pragma unroll
-        for (int i = 0; i < int(kSpecies); ++i) c.sca[i] = i < kAer ? at[(1 + i) * kWaveThreads] : 0.0f;
-        c.scattering = at[(1 + kAer) * kWaveThreads];
-        c.abs_total = 0.0f;
-        c.extinction = c.scattering;
-        return c;
-    }
+__host__ __device__ constexpr uint32_t path_rows() {
+    return kAer == 1 ? 7u : 9u;
+}
+
+// The stage queues of a block: rings of path numbers with counters of what was
+// ever taken (head) and put (tail).  A slot holds kEmpty unless a path number
+// is waiting in it.
+constexpr uint32_t kEmpty = 0xffffu;
+struct Queues {
+    uint32_t head[kQueues];
+    uint32_t tail[kQueues];
+    uint32_t live;   // paths that may still have work
+    uint32_t _pad[3];
 };
 
-// Byte offset of the vertex cache in the dynamic shared memory (after the
-// staged medium tables) and the block's total dynamic shared memory.
-__host__ __device__ inline size_t vertex_cache_offset(uint32_t knots, uint32_t bands) {
-    return (staged_medium_bytes(knots, bands) + 15u) & ~size_t(15u);
+__host__ __device__ inline uint32_t queue_slots(uint32_t paths) {
+    uint32_t n = 32u;
+    while (n < paths) n <<= 1;
+    return n;
 }
-__host__ __device__ inline size_t wave_smem_bytes(uint32_t knots, uint32_t bands, uint32_t aerosol_species) {
-    return vertex_cache_offset(knots, bands) + size_t(2u + aerosol_species) * kWaveThreads * sizeof(float);
+
+__host__ __device__ inline size_t align16(size_t v) { return (v + 15u) & ~size_t(15u); }
+__host__ __device__ inline size_t pool_offset(uint32_t knots, uint32_t bands) {
+    return align16(staged_medium_bytes(knots, bands));
+}
+// Dynamic shared memory of a block: staged medium, paths, queues.
+template <int kAer>
+__host__ __device__ inline size_t wave_smem_bytes(uint32_t knots, uint32_t bands, uint32_t paths) {
+    return pool_offset(knots, bands) + size_t(paths) * path_rows<kAer>() * 16u + sizeof(Queues) +
+           size_t(kQueues) * queue_slots(paths) * sizeof(uint16_t);
+}
+
+// Orders a warp's accesses to paths before (after) it puts them into (takes
+// them from) a queue.
+__device__ __forceinline__ void fence_block() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+
+__device__ __forceinline__ float as_f(uint32_t v) { return __uint_as_float(v); }
+__device__ __forceinline__ uint32_t as_u(float v) { return __float_as_uint(v); }
+
+__device__ __forceinline__ Rng path_rng(const float4& C, uint32_t dim) {
+    Rng r;
+    r.k0 = as_u(C.x);
+    r.k1 = as_u(C.y);
+    r.k2 = (as_u(C.z) & 255u) * 1664525u + 1013904223u;
+    r.dim = dim;
+    return r;
+}
+
+// Start of a ray's tracking: what of the tracker's state depends on the ray
+// alone, and the first draws.  Fills B and the layer bits of C.z.
+template <int kTracking>
+__device__ __forceinline__ void track_begin(const DevScene& S, const RayGeo& g, float t_max, uint32_t band, Rng& rng,
+                                            float4& B, uint32_t& meta, Counters& n) {
+    if constexpr (kTracking == SKY_TRACKING_MERGED_LAYERS) {
+        const MergedGrid G = merged_grid(S, band);
+        int m = merged_layer_at(S, G, altitude_at(g, fminf(kRayEpsilonKm, t_max), S.ground_radius));
+        int dir;
+        const float t_seg = merged_crossing(G, g, m, 0.0f, t_max, dir);
+        ++n.e[SKY_EVENT_SEGMENT];
+        const float tau = -__logf(fmaxf(1.0f - rng.next(), 0.0000001f));
+        B = make_float4(0.0f, tau, t_seg, as_f(rng.dim));
+        meta |= (uint32_t(m) << 16) | (uint32_t(dir + 1) << 28);
+    } else {
+        B = make_float4(0.0f, -1.0f, as_f(0u), as_f(rng.dim));  // no optical depth drawn, no segment behind it
+    }
+}
+
+// Track the warp's rays until at most `park` of them are under way.  Returns
+// how the lane's ray ended (0: not yet), with t at its end.
+template <int kTracking>
+__device__ __forceinline__ uint32_t track_batch(const DevScene& S, const Medium& M, bool alive, const RayGeo& g,
+                                                float t_max, uint32_t band, bool shadow, Rng& rng, float4& B,
+                                                uint32_t& meta, Counters& n, bool& watchdog, uint32_t park) {
+    const float2* sig_row = S.sigma_t + band * S.knot_count;
+    const float4* cell_row = S.sig_cell + band * kFinderCells;
+    float t = B.x;
+    uint32_t ended = 0u;
+    if constexpr (kTracking == SKY_TRACKING_MERGED_LAYERS) {
+        // track_ray_merged: a step is one crossing at most, then one tentative collision
+        // at most (two crossings a step: +1 %)
+        const MergedGrid G = merged_grid(S, band);
+        int m = int((meta >> 16) & 0xfffu), dir = int(meta >> 28) - 1;
+        float tau = B.y, t_seg = B.z;
+        float maj = alive ? __ldg(G.maj + m) : 1.0f;
+        for (uint32_t step = 0u; step < 4096u; ++step) {  // a ray crosses at most 2 x 1024 shells
+            // the next tentative collision: one expression, which the compiler contracts into
+            // the multiply-add that the plain kernel rounds with
+            float next_t = 0.0f;
+            if (alive) {
+                next_t = t + tau / maj;
+                if (!(next_t < t_seg)) {
+                    if (dir == 0) {
+                        ended = kMiss;
+                        alive = false;
+                    } else {
+                        tau = fmaxf(tau - (t_seg - t) * maj, 0.0f);
+                        t = t_seg;
+                        m += dir;
+                        t_seg = merged_crossing(G, g, m, t, t_max, dir);
+                        maj = __ldg(G.maj + m);
+                        ++n.e[SKY_EVENT_SEGMENT];
+                        next_t = t + tau / maj;
+                    }
+                }
+            }
+            if (alive && next_t < t_seg) {
+                t = next_t;
+                ++n.e[SKY_EVENT_TRACK_STEP];
+                const float accept = rng.next() * maj;
+                const float sig =
+                    sigma_t_at(S, M.knot_z, M.finder, sig_row, cell_row, altitude_at(g, t, S.ground_radius));
+                if (accept < sig) {
+                    ended = kHit;
+                    alive = false;
+                } else {
+                    tau = -__logf(fmaxf(1.0f - rng.next(), 0.0000001f));
+                }
+            }
+            if (uint32_t(__popc(__ballot_sync(kFull, alive))) <= park) break;
+        }
+        B.x = t;
+        B.y = tau;
+        B.z = t_seg;
+        meta = (meta & 0xffffu) | (uint32_t(m) << 16) | (uint32_t(dir + 1) << 28);
+    } else {
+        // track_ray's other modes: a step opens a segment if the ray is at one's
+        // start, and makes one draw in it; rays park at a segment's start only
+        const float* maj_row = S.majorants + band * S.layer_count;
+        float tau = B.y, seg_end = 0.0f, maj = 1.0f;
+        uint32_t guard = as_u(B.z);
+        bool open = false;
+        for (;;) {
+            // segment restart: the step's draw, made before its segment is known so that the
+            // two chains of arithmetic overlap; it counts (dim) only where it is used
+            Rng ahead = rng;
+            float lg = 0.0f;
+            if constexpr (kTracking == SKY_TRACKING_SEGMENT_RESTART)
+                lg = __logf(fmaxf(1.0f - ahead.next(), 0.0000001f));
+            if (alive && !open) {
+                if (t >= t_max) {
+                    ended = kMiss;
+                    alive = false;
+                } else if (guard > 100000u) {
+                    watchdog = true;
+                    ended = shadow ? kHit : kMiss;
+                    alive = false;
+                } else {
+                    ++guard;
+                    uint32_t layer;
+                    seg_end = next_segment_end(S, g, t, t_max, layer);
+                    ++n.e[SKY_EVENT_SEGMENT];
+                    maj = fmaxf(__ldg(maj_row + layer), 0.00000001f);
+                    open = true;
+                }
+            }
+            if (alive) {
+                bool inside;
+                if constexpr (kTracking == SKY_TRACKING_RESIDUAL_CARRY) {
+                    if (tau < 0.0f) tau = -__logf(fmaxf(1.0f - rng.next(), 0.0000001f));
+                    const float dt = tau / maj;
+                    inside = !(t + dt >= seg_end);
+                    if (inside) {
+                        t = t + dt;
+                        tau = -1.0f;
+                    } else {
+                        tau = fmaxf(tau - (seg_end - t) * maj, 0.0f);
+                    }
+                } else {
+                    inside = !(t >= seg_end);
+                    if (inside) {
+                        rng.dim = ahead.dim;
+                        t = t - lg / maj;
+                        inside = !(t >= seg_end);
+                    }
+                }
+                if (inside) {
+                    ++n.e[SKY_EVENT_TRACK_STEP];
+                    const float accept = rng.next() * maj;
+                    const float sig =
+                        sigma_t_at(S, M.knot_z, M.finder, sig_row, cell_row, altitude_at(g, t, S.ground_radius));
+                    if (accept < sig) {
+                        ended = kHit;
+                        alive = false;
+                    }
+                } else {
+                    t = seg_end;
+                    open = false;
+                }
+            }
+            const uint32_t active = __ballot_sync(kFull, alive);
+            if (uint32_t(__popc(active)) <= park && __ballot_sync(kFull, alive && open) == 0u) break;
+        }
+        B.x = t;
+        B.y = tau;
+        B.z = as_f(guard);
+    }
+    if (ended) B.y = as_f(ended);
+    B.w = as_f(rng.dim);
+    return ended;
+}
+
+// The outgoing ray of a vertex or camera (sky_trace.wgsl:709-717): false when
+// the chain ends here.
+template <int kTracking>
+__device__ __forceinline__ bool primary_ray(const DevScene& S, const DevLaunch& JL, V3 org, V3 dir, uint32_t depth,
+                                            uint32_t band, Rng& rng, float& rad, float4& A, float4& B, uint32_t& meta,
+                                            Counters& n, bool& watchdog) {
+    if (depth >= JL.watchdog_limit) {
+        watchdog = true;
+        return false;
+    }
+    const RayGeo g = ray_geo(org, dir);
+    ++n.e[SKY_EVENT_BOUNDARY];
+    float t_max;
+    uint32_t boundary;
+    if ((JL.max_orders != 0u && depth >= JL.max_orders) || !next_boundary(S, g, t_max, boundary)) {
+        rad = fmaxf(rad, 0.0f);
+        return false;
+    }
+    meta = band | (boundary == 1u ? uint32_t(kFlagTop) : 0u);
+    track_begin<kTracking>(S, g, t_max, band, rng, B, meta, n);
+    A = make_float4(g.b, g.p, g.r0sq, t_max);
+    return true;
 }
 
 // kCount: count events (SkyDeviceOutputs.counters given).  Without it the
-// counters are never read, so their increments compile away (the registers
-// they would hold are worth ~5 % at 64 registers per lane).
+// counters are never read, so their increments compile away.
 // kAer: aerosol species evaluated by the medium functions (1 or kSpecies,
 // coefficients_at()).
-template <int kTracking, int kPhase, int kMinBlocks, bool kSingle, bool kCount, int kAer>
-__global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
+template <int kTracking, int kPhase, int kWarps, bool kSingle, bool kCount, int kAer>
+__global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     wave_kernel(const __grid_constant__ DevScene S, const __grid_constant__ DevLaunch L0,
-                const DevJob* __restrict__ jobs, uint32_t num_jobs,
-                uint32_t total_cells, uint32_t* __restrict__ work_counter, unsigned long long* __restrict__ counters,
-                uint32_t* __restrict__ status, uint32_t iteration_limit) {
-    extern __shared__ __align__(16) unsigned char medium_smem[];
-    const Medium M = stage_medium(S, medium_smem);
-    const VertexCoeffCache<kAer> vc{
-        reinterpret_cast<float*>(medium_smem + vertex_cache_offset(S.knot_count, S.band_count)) + threadIdx.x};
+                const DevJob* __restrict__ jobs, uint32_t num_jobs, unsigned long long total_chains, uint32_t paths,
+                uint32_t used_paths, unsigned long long* __restrict__ work_counter,
+                unsigned long long* __restrict__ counters, uint32_t* __restrict__ status, uint64_t batch_limit) {
+    constexpr uint32_t kRows = path_rows<kAer>();
+    extern __shared__ __align__(16) unsigned char smem[];
+    float4* const pool = reinterpret_cast<float4*>(smem + pool_offset(S.knot_count, S.band_count));
+    Queues* const Q = reinterpret_cast<Queues*>(pool + size_t(paths) * kRows);
+    volatile uint16_t* const slots = reinterpret_cast<volatile uint16_t*>(Q + 1);
+    const uint32_t ring = queue_slots(paths), mask = ring - 1u;
     const uint32_t lane = threadIdx.x & 31u;
+    // every path starts without a chain, in the start queue
+    for (uint32_t i = threadIdx.x; i < kQueues * ring; i += blockDim.x)
+        slots[i] = uint16_t(i >= kQStart * ring && i < kQStart * ring + used_paths ? i - kQStart * ring : kEmpty);
+    for (uint32_t i = threadIdx.x; i < used_paths; i += blockDim.x)
+        pool[i * kRows + kB] = make_float4(0.0f, as_f(kFresh), 0.0f, 0.0f);
+    if (threadIdx.x < kQueues) {
+        Q->head[threadIdx.x] = 0u;
+        Q->tail[threadIdx.x] = threadIdx.x == kQStart ? used_paths : 0u;
+    }
+    if (threadIdx.x == 0u) Q->live = used_paths;
+    const Medium M = stage_medium(S, smem);  // ends with the block's only barrier
     Counters n;
     n.clear();
     bool watchdog = false;
-    // the warp's current cell and its next unclaimed sample (warp-uniform)
-    uint32_t claim_job = 0u, claim_spp = 0u, claim_next = 0u;
-    uint32_t claim_band = 0u, claim_x = 0u, claim_y = 0u;  // the cell's band and pixel, divided out once per cell
-    bool exhausted = false;
-    // the lane's chain
-    uint32_t next = kIdle, job = 0u, sample = 0u, band = 0u, px = 0u, py = 0u, depth = 0u, ls = 0u, boundary = 0u;
-    bool shadow_ray = false, ground = false;
-    Rng rng;
-    rng.k0 = rng.k1 = rng.k2 = rng.dim = 0u;
-    V3 org = mk(0.0f, 0.0f, 0.0f), dir = org;  // org is the vertex position between rays
-    // nee_mu: the pending shadow ray's cosine (to the incoming direction at a
-    // medium vertex, to the normal on the ground); its NEE term is evaluated
-    // after the trace, and only when the ray reaches the sun
-    float thr = 0.0f, rad = 0.0f, nee = 0.0f, alt = 0.0f, nee_mu = 0.0f, t_max = 0.0f;
-    RayGeo g{0.0f, 0.0f, 0.0f};
-    // FP64 sums of the lane's current cell
-    uint32_t acc_job = 0u, acc_cell = kNoCell;
-    double acc_sum = 0.0, acc_sq = 0.0;
+    uint32_t idle = 0u, turn = (threadIdx.x >> 5) & 3u;
 
-    for (uint32_t iter = 0u;; ++iter) {
-        if (iter >= iteration_limit) {  // warp-uniform
+    for (uint64_t batch = 0u;;) {
+        // the fullest queue: lanes 0-3 look at one each.  A lane's head, read before its
+        // tail, goes with its own count: the exchange below fails if the head has moved
+        // since, so what it takes has been put there.
+        uint32_t h = 0u, count = 0u;
+        if (lane < kQueues) {
+            h = *reinterpret_cast<volatile uint32_t*>(&Q->head[lane]);
+            count = *reinterpret_cast<volatile uint32_t*>(&Q->tail[lane]) - h;
+        }
+        // a full batch if there is one, of the warp's last stage rather than of another:
+        // warps that stay with a stage keep its code in the instruction caches (fullest
+        // queue first: +8 %, stages in turn: +4 %); else the fullest queue
+        const uint32_t full = __ballot_sync(kFull, count >= 32u);
+        uint32_t stage, waiting = 32u;
+        if (full) {
+            stage = (uint32_t(__ffs(int((full | (full << 4)) >> turn))) - 1u + turn) & 3u;
+            turn = stage;
+        } else {
+            const uint32_t best = __reduce_max_sync(kFull, (count << 2) | (lane & 3u));
+            stage = best & 3u;
+            waiting = best >> 2;
+        }
+        if (waiting == 0u) {
+            // one lane looks for all: the warp leaves together
+            if (__shfl_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&Q->live), 0) == 0u) break;
+            if (++idle >= kMaxIdlePolls) {
+                if (lane == 0u) atomicOr(status, 2u);
+                break;
+            }
+            __nanosleep(100);
+            __syncwarp();
+            continue;
+        }
+        if (batch >= batch_limit) {  // warp-uniform
             if (lane == 0u) atomicOr(status, 2u);
             break;
         }
-        // a chain that ended after its last ray: its radiance joins the cell's sums
-        if (next == kEnd) {
-            const double rd = double(rad);
-            acc_sum += rd;
-            acc_sq += rd * rd;
-            next = kIdle;
-        }
-        // idle lanes take the next samples of the warp's cell
-#pragma unroll 1
-        for (;;) {
-            const uint32_t need = __ballot_sync(kFull, next == kIdle);
-            if (need == 0u || exhausted) break;
-            if (claim_next >= claim_spp) {
-                uint32_t gc = 0u;
-                if (lane == 0u) gc = atomicAdd(work_counter, 1u);
-                gc = __shfl_sync(kFull, gc, 0);
-                if (gc >= total_cells) {
-                    exhausted = true;
-                    break;
-                }
-                claim_job = job_of(jobs, num_jobs, gc);
-                const uint32_t c = gc - __ldg(&jobs[claim_job].cell_begin);
-                // claims run band-major (all pixels of a band, then the next band), so the
-                // warps of an SM work on one or two bands at a time and that band's
-                // extinction row, merged grid and phase rows stay in L1 (-0.9 % on the
-                // production render, -4 % on a 128x64 one); the sums keep their
-                // pixel-major, band-minor layout
-                const uint32_t width = __ldg(&jobs[claim_job].L.width);
-                const uint32_t npix = width * __ldg(&jobs[claim_job].L.rows);
-                claim_band = c / npix;
-                const uint32_t pixel = c - claim_band * npix;
-                const uint32_t row = pixel / width;  // row within the job's slab
-                claim_x = pixel - row * width;
-                claim_y = row + __ldg(&jobs[claim_job].L.row_begin);
-                claim_spp = __ldg(&jobs[claim_job].L.spp);
-                claim_next = 0u;
+        const uint32_t take = min(waiting, 32u);
+        h = __shfl_sync(kFull, h, stage);
+        uint32_t seen = 0u;
+        if (lane == 0u) seen = atomicCAS(&Q->head[stage], h, h + take);
+        if (__shfl_sync(kFull, seen, 0) != h) continue;  // another warp was first
+        ++batch;
+        const bool on = lane < take;
+        uint32_t id = 0u;
+        if (on) {
+            volatile uint16_t* slot = slots + stage * ring + ((h + lane) & mask);
+            uint32_t v = *slot, polls = 0u;
+            while (v == kEmpty && ++polls < kMaxSlotPolls) v = *slot;  // put, but not yet written
+            *slot = uint16_t(kEmpty);
+            id = v;
+            if (v == kEmpty) {
+                atomicOr(status, 2u);
+                id = 0u;
             }
-            const uint32_t rank = __popc(need & ((1u << lane) - 1u));
-            if (next == kIdle && claim_next + rank < claim_spp) {
-                job = claim_job;
-                band = claim_band;
-                px = claim_x;
-                py = claim_y;
-                sample = claim_next + rank;
-                next = kStart;
-            }
-            claim_next = min(claim_spp, claim_next + uint32_t(__popc(need)));
         }
-        // event code up to the lane's next ray, one pass in flow order (start,
-        // lights / continuation, outgoing ray), so that each block runs once
-        // per iteration for every lane that needs it
-        if (next != kIdle && next != kTrace) {
-            const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
-            if (next == kStart) {
-                // the image pixel drives the random stream, the slab pixel indexes the sums
-                const uint32_t pixel = py * JL.width + px;
-                const uint32_t cell = ((py - JL.row_begin) * JL.width + px) * S.band_count + band;
-                if (cell != acc_cell || job != acc_job) {
-                    if (acc_cell != kNoCell) {
-                        const DevJob& A = jobs[acc_job];
-                        atomicAdd(A.cell_sum + acc_cell, acc_sum);
-                        double* sq = A.cell_sumsq;
-                        if (sq) atomicAdd(sq + acc_cell, acc_sq);
+        fence_block();
+        float4* const P = pool + id * kRows;
+        uint32_t next = kQNone;
+        // the lane's ray: set up by its stage, or taken up where it was left
+        bool tracing = false;
+        float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = A;
+        uint32_t meta = 0u;
+        Rng rng;
+        rng.k0 = rng.k1 = rng.k2 = rng.dim = 0u;
+
+        if (stage == kQTrack) {
+            if (on) {
+                A = P[kA];
+                B = P[kB];
+                const float4 C = P[kC];
+                meta = as_u(C.z);
+                rng = path_rng(C, as_u(B.w));
+                tracing = true;
+            }
+        } else if (stage == kQVertex) {
+            if (on) {
+                A = P[kA];
+                B = P[kB];
+                const float4 C = P[kC], D = P[kD], E = P[kE];
+                meta = as_u(C.z);
+                const uint32_t band = meta & 255u, job = as_u(C.w) & 0xffffu;
+                uint32_t ls = as_u(C.w) >> 16;
+                const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
+                V3 org = mk(D.x, D.y, D.z);
+                const V3 dir = mk(E.x, E.y, E.z);
+                bool ground = (meta & kFlagGround) != 0u, alive = true;
+                if (!(meta & kFlagShadow)) {  // a new vertex
+                    ls = 0u;
+                    float thr = D.w;
+                    ground = as_u(B.y) != kHit;
+                    if (!ground) {
+                        const RayGeo g{A.x, A.y, A.z};
+                        org = madd(org, dir, B.x);
+                        const float alt = altitude_at(g, B.x, S.ground_radius);
+                        ++n.e[SKY_EVENT_SCATTER];
+                        const Coeffs c = coefficients_at<kAer>(S, M, band, alt);
+                        const bool medium = c.extinction > 0.0f && c.scattering > 0.0f;
+                        if (medium) thr *= fminf(fmaxf(c.scattering / c.extinction, 0.0f), 1.0f);
+                        if (!medium || thr <= 0.0f) {
+                            alive = false;
+                        } else {
+                            P[kG] = make_float4(c.rayleigh, c.scattering, c.sca[0], c.sca[1]);
+                            if (kAer > 1) P[kH] = make_float4(c.sca[2], c.sca[3], 0.0f, 0.0f);
+                        }
+                    } else {
+                        ++n.e[SKY_EVENT_GROUND];
+                        org = madd(org, dir, A.w);
                     }
-                    acc_job = job;
-                    acc_cell = cell;
-                    acc_sum = acc_sq = 0.0;
+                    P[kD] = make_float4(org.x, org.y, org.z, thr);
+                    reinterpret_cast<float*>(&P[kF])[2] = 0.0f;  // the vertex's NEE sum
                 }
-                rng.init(pixel, JL.sample_offset + sample, band, JL.seed_lo, JL.seed_hi);
-                dir = camera_dir(JL, px, py, rng);
-                org = mk(0.0f, S.ground_radius + fmaxf(JL.observer_altitude, 0.0f), 0.0f);
-                ++n.e[SKY_EVENT_CHAIN];
-                thr = 1.0f;
-                rad = 0.0f;
-                depth = 0u;
-                next = kPrimary;
+                if (!alive) {
+                    reinterpret_cast<float*>(&P[kE])[3] = fmaxf(E.w, 0.0f);
+                    reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
+                    next = kQStart;
+                } else {
+                    // direct_sun_at_scatter (sky_trace.wgsl:566-585) and ground_radiance
+                    // (:587-608), one shadow ray at a time
+                    rng = path_rng(C, as_u(B.w));
+                    const uint32_t lights = JL.direct_light_samples;
+                    bool lit = false;
+                    meta = band | kFlagShadow | (ground ? uint32_t(kFlagGround) : 0u);
+                    RayGeo g;
+                    float t_max = 0.0f, nee_mu = 0.0f;
+                    while (ls < lights) {
+                        ++ls;
+                        const V3 ldir = sample_sun_cone(job_scene<kSingle>(S, jobs, job), rng);
+                        ++n.e[SKY_EVENT_NEE];
+                        float cos_sun = 0.0f;
+                        if (ground) {
+                            cos_sun = fmaxf(dot3(normalize_or_y(org), ldir), 0.0f);
+                            if (!(cos_sun > 0.0f)) continue;
+                        }
+                        g = ray_geo(madd(org, ldir, kRayEpsilonKm), ldir);
+                        uint32_t kind;
+                        ++n.e[SKY_EVENT_BOUNDARY];
+                        if (!(next_boundary(S, g, t_max, kind) && kind == 1u)) continue;
+                        nee_mu = ground ? cos_sun : dot3(dir, ldir);
+                        lit = true;
+                        break;
+                    }
+                    if (lit) {
+                        track_begin<kTracking>(S, g, t_max, band, rng, B, meta, n);
+                        A = make_float4(g.b, g.p, g.r0sq, t_max);
+                        reinterpret_cast<float*>(&P[kF])[3] = nee_mu;
+                        tracing = true;
+                    } else {
+                        // no sun: as a shadow ray that collides
+                        P[kB] = make_float4(0.0f, as_f(kHit), 0.0f, as_f(rng.dim));
+                        reinterpret_cast<float*>(&P[kC])[2] = as_f(meta);
+                        next = kQContinue;
+                    }
+                    reinterpret_cast<float*>(&P[kC])[3] = as_f(job | (ls << 16));
+                }
             }
-            if (next == kLights) {
-                // direct_sun_at_scatter (sky_trace.wgsl:566-585) and ground_radiance
-                // (:587-608), one shadow ray at a time
+        } else if (stage == kQContinue) {
+            if (on) {
+                const float4 C = P[kC], D = P[kD], E = P[kE], F = P[kF];
+                B = P[kB];
+                meta = as_u(C.z);
+                const uint32_t band = meta & 255u, job = as_u(C.w) & 0xffffu, ls = as_u(C.w) >> 16;
+                const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
+                const bool ground = (meta & kFlagGround) != 0u;
+                V3 org = mk(D.x, D.y, D.z), dir = mk(E.x, E.y, E.z);
+                float nee = F.z;
+                Coeffs c;
+                if (!ground) {
+                    const float4 G = P[kG];
+                    c.rayleigh = G.x;
+                    c.scattering = G.y;
+                    c.sca[0] = G.z;
+                    c.sca[1] = c.sca[2] = c.sca[3] = 0.0f;
+                    if (kAer > 1) {
+                        const float4 H = P[kH];
+                        c.sca[1] = G.w;
+                        c.sca[2] = H.x;
+                        c.sca[3] = H.y;
+                    }
+                    c.abs_total = 0.0f;
+                    c.extinction = c.scattering;
+                }
+                if (as_u(B.y) == kMiss) {  // the sample's term, transmittance 1 (sky_trace.wgsl:566-608)
+                    const float l_sun = M.bands[band].solar_radiance;
+                    const float nee_mu = F.w;
+                    nee += ground ? S.ground_albedo * kInvPi * l_sun * 1.0f * nee_mu / S.light_pdf
+                                  : l_sun * 1.0f * mixed_phase<kAer>(S, c, band, nee_mu) / S.light_pdf;
+                }
                 const uint32_t lights = JL.direct_light_samples;
-                while (ls < lights) {
-                    ++ls;
-                    const V3 ldir = sample_sun_cone(job_scene<kSingle>(S, jobs, job), rng);
-                    ++n.e[SKY_EVENT_NEE];
-                    float cos_sun = 0.0f;
-                    if (ground) {
-                        cos_sun = fmaxf(dot3(normalize_or_y(org), ldir), 0.0f);
-                        if (!(cos_sun > 0.0f)) continue;
-                    }
-                    g = ray_geo(madd(org, ldir, kRayEpsilonKm), ldir);
-                    uint32_t kind;
-                    ++n.e[SKY_EVENT_BOUNDARY];
-                    if (!(next_boundary(S, g, t_max, kind) && kind == 1u)) continue;
-                    nee_mu = ground ? cos_sun : dot3(dir, ldir);
-                    shadow_ray = true;
-                    next = kTrace;
-                    break;
-                }
-                if (next == kLights) {
+                if (ls < lights) {
+                    reinterpret_cast<float*>(&P[kF])[2] = nee;
+                    next = kQVertex;
+                } else {
                     // the continuation (sky_trace.wgsl:728-767): each branch draws its
                     // angles, then one shared frame step turns them into the direction
                     // (orthonormal_basis + direction_from_frame, as direction_from_axis_mu
                     // and sample_cosine_hemisphere compute it), so that medium and ground
                     // lanes run that step together
+                    rng = path_rng(C, as_u(B.w));
+                    float thr = D.w, rad = E.w;
+                    uint32_t depth = as_u(F.x);
                     rad += thr * (nee * (1.0f / float(lights)));
                     V3 nd = mk(0.0f, 1.0f, 0.0f), axis = dir;
                     float cos_t = 1.0f, sin_t = 0.0f, xi_phi = 0.0f, weight = 1.0f;
                     bool framed = true;
                     if (!ground) {
-                        const Coeffs c = vc.load();
                         if (kPhase == SKY_PHASE_TABULATED) {
                             float mu;
                             weight = tabulated_mu<kAer>(S, c, band, rng, mu, xi_phi);
@@ -324,16 +570,16 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
                         xi_phi = rng.next();
                         cos_t = sqrtf(fmaxf(1.0f - u, 0.0f));
                     }
-                    V3 n = axis;
+                    V3 nrm = axis;
                     if (framed) {
                         V3 t, bt;
                         orthonormal_basis(axis, t, bt);
-                        n = normalize_or_y(axis);
-                        nd = direction_from_frame(n, t, bt, cos_t, sin_t, xi_phi);
+                        nrm = normalize_or_y(axis);
+                        nd = direction_from_frame(nrm, t, bt, cos_t, sin_t, xi_phi);
                     }
                     bool alive = true;
                     if (ground) {
-                        const float pdf = fmaxf(dot3(n, nd), 0.0f) * kInvPi;
+                        const float pdf = fmaxf(dot3(nrm, nd), 0.0f) * kInvPi;
                         const float cos_out = fmaxf(dot3(axis, nd), 0.0f);
                         if (pdf <= 0.0f || cos_out <= 0.0f) alive = false;
                         else thr *= S.ground_albedo * kInvPi * cos_out / pdf;
@@ -347,101 +593,143 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
                     }
                     if (!alive) {
                         rad = fmaxf(rad, 0.0f);
-                        next = kEnd;
                     } else {
                         org = madd(org, nd, kRayEpsilonKm);
                         dir = nd;
                         if (rad < 0.0f || rad != rad || thr < 0.0f || thr != thr) {
                             rad = 0.0f;
-                            next = kEnd;
+                            alive = false;
                         } else {
                             ++depth;
-                            next = kPrimary;
                         }
                     }
-                }
-            }
-            if (next == kPrimary) {  // the outgoing ray (sky_trace.wgsl:709-717)
-                const uint32_t max_orders = JL.max_orders;
-                if (depth >= JL.watchdog_limit) {
-                    watchdog = true;
-                    next = kEnd;
-                } else {
-                    g = ray_geo(org, dir);
-                    ++n.e[SKY_EVENT_BOUNDARY];
-                    if ((max_orders != 0u && depth >= max_orders) || !next_boundary(S, g, t_max, boundary)) {
-                        rad = fmaxf(rad, 0.0f);
-                        next = kEnd;
+                    if (alive)
+                        alive = primary_ray<kTracking>(S, JL, org, dir, depth, band, rng, rad, A, B, meta, n, watchdog);
+                    if (alive) {
+                        P[kD] = make_float4(org.x, org.y, org.z, thr);
+                        P[kE] = make_float4(dir.x, dir.y, dir.z, rad);
+                        reinterpret_cast<float*>(&P[kF])[0] = as_f(depth);
+                        tracing = true;
                     } else {
-                        shadow_ray = false;
-                        next = kTrace;
+                        reinterpret_cast<float*>(&P[kE])[3] = rad;
+                        reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
+                        next = kQStart;
                     }
                 }
             }
-        }
-        const bool tracing = next == kTrace;
-        if (!__any_sync(kFull, tracing)) {
-            // no cell left and every lane idle (a lane ending its chain is summed next
-            // iteration)
-            if (exhausted && __all_sync(kFull, next == kIdle)) break;
-            continue;
-        }
-        if (tracing) {
-            float t_hit = 0.0f;
-            const bool hit = track_ray<kTracking>(S, M, g, t_max, band, rng, t_hit, n, watchdog, shadow_ray);
-            // the medium coefficients at a real collision (albedo; kept for the new
-            // vertex's NEE terms and continuation) and at the vertex of an unblocked
-            // shadow ray (phase of its NEE term, from the vertex cache)
-            const bool lit = shadow_ray && !hit;
-            Coeffs c;
-            if (!shadow_ray && hit) {
-                org = madd(org, dir, t_hit);
-                alt = altitude_at(g, t_hit, S.ground_radius);
-                c = coefficients_at<kAer>(S, M, band, alt);
-                vc.store(c);
-            } else if (lit && !ground) {
-                c = vc.load();
-            }
-            if (shadow_ray) {
-                if (lit) {  // the sample's term, transmittance 1 (sky_trace.wgsl:566-608)
-                    const float l_sun = M.bands[band].solar_radiance;
-                    nee += ground ? S.ground_albedo * kInvPi * l_sun * 1.0f * nee_mu / S.light_pdf
-                                  : l_sun * 1.0f * mixed_phase<kAer>(S, c, band, nee_mu) / S.light_pdf;
-                }
-                next = kLights;
-            } else if (hit) {
-                ++n.e[SKY_EVENT_SCATTER];
-                const bool medium = c.extinction > 0.0f && c.scattering > 0.0f;
-                if (medium) thr *= fminf(fmaxf(c.scattering / c.extinction, 0.0f), 1.0f);
-                if (!medium || thr <= 0.0f) {
+        } else {
+            // the chains that ended
+            float rad = 0.0f;
+            uint32_t old_cell = 0u, old_job = 0u;
+            const uint32_t state = on ? as_u(P[kB].y) : uint32_t(kFresh);
+            if (state != kFresh) {
+                const float4 C = P[kC], E = P[kE], F = P[kF];
+                rad = E.w;
+                old_cell = as_u(F.y);
+                old_job = as_u(C.w) & 0xffffu;
+                if (state == kMiss) {  // left through the top of the atmosphere
+                    if (as_u(F.x) == 0u && dot3(mk(E.x, E.y, E.z), load3(job_scene<kSingle>(S, jobs, old_job).sun)) >=
+                                               S.cos_max)
+                        rad += P[kD].w * M.bands[as_u(C.z) & 255u].solar_radiance;
                     rad = fmaxf(rad, 0.0f);
-                    next = kEnd;
-                } else {
-                    ground = false;
-                    ls = 0u;
-                    nee = 0.0f;
-                    next = kLights;
                 }
-            } else if (boundary == 1u) {
-                if (depth == 0u && dot3(dir, load3(job_scene<kSingle>(S, jobs, job).sun)) >= S.cos_max)
-                    rad += thr * M.bands[band].solar_radiance;
-                rad = fmaxf(rad, 0.0f);
-                next = kEnd;
-            } else {
-                ++n.e[SKY_EVENT_GROUND];
-                org = madd(org, dir, t_max);
-                ground = true;
-                ls = 0u;
-                nee = 0.0f;
-                next = kLights;
+            }
+            // the next samples of the launch, band-major (all pixels of a band, then the
+            // next band), so that the warps of the chip work on one or two bands at a
+            // time and that band's extinction row, merged grid and phase rows stay in L1;
+            // the sums keep their pixel-major, band-minor layout
+            unsigned long long base = 0u;
+            if (lane == 0u) base = atomicAdd(work_counter, (unsigned long long)take);
+            base = __shfl_sync(kFull, base, 0);
+            const unsigned long long at = base + lane;
+            const bool more = on && at < total_chains;
+            if (more) {
+                uint32_t job = 0u;
+                if constexpr (!kSingle) {  // the last job whose first chain is <= at
+                    uint32_t hi = num_jobs;
+                    while (hi - job > 1u) {
+                        const uint32_t mid = (job + hi) >> 1;
+                        if (__ldg(&jobs[mid].chain_begin) <= at) job = mid;
+                        else hi = mid;
+                    }
+                }
+                const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
+                const unsigned long long rel = kSingle ? at : at - __ldg(&jobs[job].chain_begin);
+                // rel / spp: the product with floor((2^64 - 1) / spp) is at most one short
+                uint32_t c = uint32_t(__umul64hi(rel, JL.spp_reciprocal));
+                uint32_t sample = uint32_t(rel - (unsigned long long)c * JL.spp);
+                if (sample >= JL.spp) {
+                    ++c;
+                    sample -= JL.spp;
+                }
+                const uint32_t npix = JL.width * JL.rows;
+                const uint32_t band = c / npix;
+                const uint32_t slab_pixel = c - band * npix;
+                const uint32_t row = slab_pixel / JL.width;  // row within the job's slab
+                const uint32_t px = slab_pixel - row * JL.width, py = row + JL.row_begin;
+                // the image pixel drives the random stream, the slab pixel indexes the sums
+                rng.init(py * JL.width + px, JL.sample_offset + sample, band, JL.seed_lo, JL.seed_hi);
+                const V3 dir = camera_dir(JL, px, py, rng);
+                const V3 org = mk(0.0f, S.ground_radius + fmaxf(JL.observer_altitude, 0.0f), 0.0f);
+                ++n.e[SKY_EVENT_CHAIN];
+                float new_rad = 0.0f;
+                meta = band;
+                tracing = primary_ray<kTracking>(S, JL, org, dir, 0u, band, rng, new_rad, A, B, meta, n, watchdog);
+                if (!tracing) {
+                    reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
+                    next = kQStart;
+                }
+                P[kC] = make_float4(as_f(rng.k0), as_f(rng.k1), as_f(meta), as_f(job));
+                P[kD] = make_float4(org.x, org.y, org.z, 1.0f);
+                P[kE] = make_float4(dir.x, dir.y, dir.z, new_rad);
+                P[kF] = make_float4(as_f(0u), as_f(slab_pixel * S.band_count + band), 0.0f, 0.0f);
+            }
+            const uint32_t gone = __popc(__ballot_sync(kFull, on && !more));
+            if (gone && lane == 0u) atomicSub(&Q->live, gone);
+            if (rad != 0.0f) {  // the sums start at zero
+                const DevJob& J = jobs[old_job];
+                const double rd = double(rad);
+                atomicAdd(J.cell_sum + old_cell, rd);
+                double* sq = J.cell_sumsq;
+                if (sq) atomicAdd(sq + old_cell, rd * rd);
             }
         }
-    }
-    if (acc_cell != kNoCell) {
-        const DevJob& A = jobs[acc_job];
-        atomicAdd(A.cell_sum + acc_cell, acc_sum);
-        double* sq = A.cell_sumsq;
-        if (sq) atomicAdd(sq + acc_cell, acc_sq);
+
+        // track the rays at once, whatever stage they come from
+        const uint32_t rays = __popc(__ballot_sync(kFull, tracing));
+        if (rays) {
+            const RayGeo g{A.x, A.y, A.z};
+            // park few rays, and fewer of a small batch
+            const uint32_t park = min(kTracking == SKY_TRACKING_MERGED_LAYERS ? kPark : kParkLayered, rays * 3u / 8u);
+            const uint32_t ended = track_batch<kTracking>(S, M, tracing, g, A.w, meta & 255u,
+                                                          (meta & kFlagShadow) != 0u, rng, B, meta, n, watchdog, park);
+            if (tracing) {
+                if (!ended) next = kQTrack;
+                else if (meta & kFlagShadow) next = kQContinue;
+                else next = ended == kMiss && (meta & kFlagTop) ? kQStart : kQVertex;
+                if (next == kQTrack || next == kQVertex) P[kA] = A;
+                P[kB] = B;
+                reinterpret_cast<float*>(&P[kC])[2] = as_f(meta);
+            }
+        }
+
+        // each path into the queue of its next stage: one lane of those that go to a queue
+        // takes room for all of them
+        const uint32_t own = __match_any_sync(kFull, next);
+        const uint32_t first = uint32_t(__ffs(int(own))) - 1u;
+        fence_block();
+        uint32_t room = 0u;
+        if (lane == first && next != kQNone) room = atomicAdd(&Q->tail[next], uint32_t(__popc(own)));
+        room = __shfl_sync(kFull, room, first);
+        if (next != kQNone) {
+            volatile uint16_t* slot =
+                slots + next * ring + ((room + __popc(own & ((1u << lane) - 1u))) & mask);
+            uint32_t polls = 0u;
+            while (*slot != kEmpty && ++polls < kMaxSlotPolls) {}  // its last path is being taken
+            if (polls >= kMaxSlotPolls) atomicOr(status, 2u);
+            *slot = uint16_t(id);
+        }
+        __syncwarp();
     }
     if (kCount) {
 #pragma unroll
@@ -455,54 +743,65 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     if (__any_sync(kFull, watchdog) && lane == 0u) atomicOr(status, 1u);
 }
 
-template <int kTracking, int kPhase, int kMinBlocks, bool kSingle, bool kCount, int kAer>
+template <int kTracking, int kPhase, int kWarps, bool kSingle, bool kCount, int kAer>
 cudaError_t launch_wave_shape(const WaveLaunch& w, cudaStream_t stream) {
     const void* k =
-        reinterpret_cast<const void*>(wave_kernel<kTracking, kPhase, kMinBlocks, kSingle, kCount, kAer>);
-    int dev = 0, sms = 0, per_sm = 0;
+        reinterpret_cast<const void*>(wave_kernel<kTracking, kPhase, kWarps, kSingle, kCount, kAer>);
+    constexpr uint32_t kThreads = kWarps * 32u;
+    int dev = 0, sms = 0, per_sm = 0, smem_sm = 0, smem_block = 0, reserved = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    // the staged medium tables and the vertex cache: 12.7 KB for 81 bands over 68 knots and one
-    // aerosol species; the largest scenes the library accepts (1024 knots, 256 bands) need 77 KB,
-    // beyond the 48 KB a launch gets without opting in
-    const size_t smem = wave_smem_bytes(w.scene.knot_count, w.scene.band_count, uint32_t(kAer));
+    if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess)
+        return e;
+    if ((e = cudaDeviceGetAttribute(&smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
+        return e;
+    if ((e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess) return e;
+    // paths of a block: a quarter more than its lanes (what waits in the queues while every
+    // warp has a batch; a half more measured the same), fewer where the scene's tables leave
+    // no room for that in two blocks per SM, in steps of 32
+    uint32_t paths = kThreads * 5u / 4u;
+    auto fits = [&](uint32_t p, int blocks) {
+        const size_t b = wave_smem_bytes<kAer>(w.scene.knot_count, w.scene.band_count, p);
+        return b <= size_t(smem_block) && size_t(blocks) * (b + size_t(reserved)) <= size_t(smem_sm);
+    };
+    while (paths > kThreads && !fits(paths, kBlocksPerSm)) paths -= 32u;
+    if (!fits(paths, kBlocksPerSm)) {
+        paths = kThreads * 5u / 4u;
+        while (paths > 32u && !fits(paths, 1)) paths -= 32u;
+    }
+    const size_t smem = wave_smem_bytes<kAer>(w.scene.knot_count, w.scene.band_count, paths);
     if (smem > 48u * 1024u &&
         (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
         return e;
-    // Prefer the smallest shared-memory carveout that holds kMinBlocks blocks' tables: the
-    // rest of the SM's L1/shared array caches the phase tables, extinction rows and merged
-    // grid (the largest carveout costs 6 % on the production render).  A hint: if the
-    // driver refuses it, the launch goes ahead with its own choice.
-    int smem_sm = 0, reserved = 0;
-    if (cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
-        smem_sm > 0) {
-        const size_t need = size_t(kMinBlocks) * (smem + size_t(reserved));
-        const int pct = int(std::min<size_t>(100u, (need * 100u + size_t(smem_sm) - 1u) / size_t(smem_sm)));
-        if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, std::max(pct, 1)) != cudaSuccess)
-            (void)cudaGetLastError();  // clear the refused hint so the launch check does not see it
-    } else {
-        (void)cudaGetLastError();
-    }
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWaveThreads, smem)) != cudaSuccess) return e;
+    // Prefer the smallest shared-memory carveout that holds two blocks: the rest of the
+    // SM's L1/shared array caches the phase tables, extinction rows and merged grid.  A
+    // hint: if the driver refuses it, the launch goes ahead with its own choice.
+    const size_t need = size_t(fits(paths, kBlocksPerSm) ? kBlocksPerSm : 1) * (smem + size_t(reserved));
+    const int pct = int(std::min<size_t>(100u, (need * 100u + size_t(smem_sm) - 1u) / size_t(smem_sm)));
+    if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, std::max(pct, 1)) != cudaSuccess)
+        (void)cudaGetLastError();  // clear the refused hint so the launch check does not see it
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem)) != cudaSuccess) return e;
     per_sm = std::max(per_sm, 1);
     if (w.max_blocks_per_sm) per_sm = std::min(per_sm, int(w.max_blocks_per_sm));
-    // a warp per cell at most
-    const uint64_t want = (uint64_t(w.total_cells) * 32u + kWaveThreads - 1u) / kWaveThreads;
+    // a warp of chains per block at least; a small render spreads its chains over the blocks
+    const uint64_t want = (w.total_chains + 31u) / 32u;
     const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * sms, want)));
-    wave_kernel<kTracking, kPhase, kMinBlocks, kSingle, kCount, kAer><<<blocks, kWaveThreads, smem, stream>>>(
-        w.scene, w.launch0, w.jobs, w.num_jobs, w.total_cells, w.work_counter, w.counters, w.status,
-        w.iteration_limit ? w.iteration_limit : kMaxIterations);
+    const uint64_t share = ((w.total_chains + blocks - 1u) / blocks + 31u) / 32u * 32u;
+    const uint32_t used = uint32_t(std::min<uint64_t>(paths, share));
+    const uint64_t limit = uint64_t(w.iteration_limit ? w.iteration_limit : kMaxIterations) * kBatchesPerIteration;
+    wave_kernel<kTracking, kPhase, kWarps, kSingle, kCount, kAer><<<blocks, kThreads, smem, stream>>>(
+        w.scene, w.launch0, w.jobs, w.num_jobs, w.total_chains, paths, used, w.work_counter, w.counters, w.status,
+        limit);
     return cudaGetLastError();
 }
 
 template <int kTracking, int kPhase, bool kSingle, bool kCount, int kAer>
 cudaError_t launch_wave_variant(const WaveLaunch& w, cudaStream_t stream) {
     switch (w.variant) {
-        case 0: return launch_wave_shape<kTracking, kPhase, 3, kSingle, kCount, kAer>(w, stream);
-        case 1: return launch_wave_shape<kTracking, kPhase, 2, kSingle, kCount, kAer>(w, stream);
-        case 2: return launch_wave_shape<kTracking, kPhase, 4, kSingle, kCount, kAer>(w, stream);
+        case 0: return launch_wave_shape<kTracking, kPhase, 12, kSingle, kCount, kAer>(w, stream);
+        case 1: return launch_wave_shape<kTracking, kPhase, 8, kSingle, kCount, kAer>(w, stream);
+        case 2: return launch_wave_shape<kTracking, kPhase, 16, kSingle, kCount, kAer>(w, stream);
         default: return cudaErrorInvalidValue;
     }
 }
