@@ -579,6 +579,18 @@ typedef struct SkyComboScore {
     double mean, rmse, p50, p90, p95, p99, max, score;
     uint64_t finite;  /* samples with a finite distance */
 } SkyComboScore;
+/*
+ * The reference of a score, on the GPU: its scale (the 99th percentile of the
+ * finite Y, element round((n - 1) 0.99), at least 1e-12; main.rs:343) unless
+ * scale_in gives one, and its Oklab at that scale, computed in FP64.
+ *   ref_xyz    device, double [samples][3]
+ *   scale_in   host, or null
+ *   ref_oklab  device, float [samples][3] (out)
+ *   scale_out  host (out)
+ * Synchronous on `cuda_stream`; device scratch is allocated per call.
+ */
+int sky_cuda_score_reference(const double* ref_xyz, uint64_t samples, const double* scale_in, float* ref_oklab,
+                             double* scale_out, void* cuda_stream);
 int sky_cuda_score_combos(const float* bands, uint32_t band_count, uint64_t samples, const float* ref_oklab,
                           float reference_scale, const uint32_t* combo_bands, const float* combo_xyz,
                           uint32_t combo_count, uint32_t channels, SkyComboScore* results, void* cuda_stream);

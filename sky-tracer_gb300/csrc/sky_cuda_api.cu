@@ -1240,6 +1240,36 @@ struct DeviceScratch {  // frees what it allocated when the call returns
 
 }  // namespace
 
+extern "C" int sky_cuda_score_reference(const double* ref_xyz, uint64_t samples, const double* scale_in,
+                                        float* ref_oklab, double* scale_out, void* cuda_stream) {
+    if (!ref_xyz || !ref_oklab || !scale_out)
+        return set_error(SKY_ERR_INVALID_CONFIG, "ref_xyz, ref_oklab and scale_out are required");
+    if (samples == 0) return set_error(SKY_ERR_INVALID_CONFIG, "samples must be positive");
+    int device = 0, sms = 1;
+    if (cudaGetDevice(&device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "no usable CUDA device");
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    DeviceScratch mem;
+    unsigned char* base = nullptr;
+    const size_t o_hist = align_up(sizeof(ScaleState), 256), bytes = o_hist + kScoreHistBins * sizeof(uint32_t);
+    cudaError_t e;
+    if ((e = mem.alloc(&base, bytes))) return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "scoring scratch allocation", e);
+    clear_stale_error();
+    ScaleState* state = reinterpret_cast<ScaleState*>(base);
+    if ((e = cudaMemsetAsync(base, 0, bytes, stream))) return cuda_fail(SKY_ERR_COPY, "scoring scratch", e);
+    if (scale_in)
+        e = cudaMemcpyAsync(&state->scale, scale_in, sizeof(double), cudaMemcpyHostToDevice, stream);
+    else
+        e = launch_reference_scale(ref_xyz, samples, state, reinterpret_cast<uint32_t*>(base + o_hist), uint32_t(sms),
+                                   stream);
+    if (e == cudaSuccess) e = launch_reference_lab(ref_xyz, samples, state, ref_oklab, stream);
+    if (e != cudaSuccess) return cuda_fail(SKY_ERR_LAUNCH, "reference kernel launch", e);
+    if ((e = cudaMemcpyAsync(scale_out, &state->scale, sizeof(double), cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaStreamSynchronize(stream)))
+        return cuda_fail(SKY_ERR_SYNC, "reference scale", e);
+    return SKY_OK;
+}
+
 extern "C" int sky_cuda_score_combos(const float* bands, uint32_t band_count, uint64_t samples,
                                      const float* ref_oklab, float reference_scale, const uint32_t* combo_bands,
                                      const float* combo_xyz, uint32_t combo_count, uint32_t channels,
@@ -1256,96 +1286,73 @@ extern "C" int sky_cuda_score_combos(const float* bands, uint32_t band_count, ui
     if (cudaGetDevice(&device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "no usable CUDA device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-    // combinations per pass: distances of at most 2^28 (1 GB) and 8192 combinations
-    const uint32_t chunk =
-        uint32_t(std::max<uint64_t>(1, std::min<uint64_t>({combo_count, 8192u, (1ull << 28) / samples})));
-    constexpr uint32_t kTargets = 5;  // p50, p90, p95, p99, max
-    const double quantiles[kTargets] = {0.50, 0.90, 0.95, 0.99, 1.0};
+    // combinations per launch sequence: as many as keep their distances (64 MB) in the L2 cache
+    // until they are selected from, one at least
+    const uint32_t chunk = uint32_t(
+        std::max<uint64_t>(1, std::min<uint64_t>({combo_count, 1024u, (uint64_t(1) << 24) / samples})));
+    // one allocation: the combinations, their states (all of them), one chunk's histograms and distances
+    size_t off = 0;
+    auto reserve = [&off](size_t bytes) {
+        const size_t at = off;
+        off = align_up(off + bytes, 256);
+        return at;
+    };
+    const size_t o_state = reserve(size_t(combo_count) * sizeof(ScoreState));
+    const size_t o_hist = reserve(size_t(chunk) * kScoreTargets * kScoreHistBins * sizeof(uint32_t));
+    const size_t cleared = off;
+    const size_t o_bands = reserve(size_t(combo_count) * channels * sizeof(uint32_t));
+    const size_t o_xyz = reserve(size_t(combo_count) * channels * 3 * sizeof(float));
+    const size_t o_dist = reserve(size_t(chunk) * samples * sizeof(float));
     DeviceScratch mem;
-    float* dist;
-    double* sums;
-    uint32_t *d_bands, *d_tcombo, *d_tprefix, *d_hist;
-    float* d_xyz;
+    unsigned char* base = nullptr;
     cudaError_t e;
-    if ((e = mem.alloc(&dist, size_t(chunk) * samples)) || (e = mem.alloc(&sums, size_t(chunk) * 3)) ||
-        (e = mem.alloc(&d_bands, size_t(chunk) * channels)) || (e = mem.alloc(&d_xyz, size_t(chunk) * channels * 3)) ||
-        (e = mem.alloc(&d_tcombo, size_t(chunk) * kTargets)) || (e = mem.alloc(&d_tprefix, size_t(chunk) * kTargets)) ||
-        (e = mem.alloc(&d_hist, size_t(chunk) * kTargets * kScoreHistBins)))
-        return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "scoring scratch allocation", e);
-    std::vector<double> h_sums(size_t(chunk) * 3);
-    std::vector<uint32_t> h_hist(size_t(chunk) * kTargets * kScoreHistBins), tcombo(size_t(chunk) * kTargets),
-        tprefix(size_t(chunk) * kTargets);
-    std::vector<uint64_t> rank(size_t(chunk) * kTargets);
+    if ((e = mem.alloc(&base, off))) return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "scoring scratch allocation", e);
     clear_stale_error();
+    if ((e = cudaMemcpyAsync(base + o_bands, combo_bands, size_t(combo_count) * channels * sizeof(uint32_t),
+                             cudaMemcpyHostToDevice, stream)) ||
+        (e = cudaMemcpyAsync(base + o_xyz, combo_xyz, size_t(combo_count) * channels * 3 * sizeof(float),
+                             cudaMemcpyHostToDevice, stream)) ||
+        (e = cudaMemsetAsync(base, 0, cleared, stream)))
+        return cuda_fail(SKY_ERR_COPY, "scoring upload", e);
     for (uint32_t c0 = 0; c0 < combo_count; c0 += chunk) {
-        const uint32_t nc = std::min(chunk, combo_count - c0);
-        if ((e = cudaMemcpyAsync(d_bands, combo_bands + size_t(c0) * channels, size_t(nc) * channels * 4,
-                                 cudaMemcpyHostToDevice, stream)) ||
-            (e = cudaMemcpyAsync(d_xyz, combo_xyz + size_t(c0) * channels * 3, size_t(nc) * channels * 12,
-                                 cudaMemcpyHostToDevice, stream)) ||
-            (e = cudaMemsetAsync(sums, 0, size_t(nc) * 3 * sizeof(double), stream)))
-            return cuda_fail(SKY_ERR_COPY, "scoring upload", e);
-        if ((e = launch_score_distances(bands, samples, ref_oklab, 1.0f / reference_scale, d_bands, d_xyz, nc,
-                                        channels, dist, sums, stream)))
-            return cuda_fail(SKY_ERR_LAUNCH, "distance kernel launch", e);
-        if ((e = cudaMemcpyAsync(h_sums.data(), sums, size_t(nc) * 3 * sizeof(double), cudaMemcpyDeviceToHost,
-                                 stream)) ||
-            (e = cudaStreamSynchronize(stream)))
-            return cuda_fail(SKY_ERR_SYNC, "distance sums", e);
-        uint32_t targets = 0;
-        for (uint32_t c = 0; c < nc; ++c) {
-            const uint64_t n = uint64_t(h_sums[c * 3 + 2] + 0.5);
-            SkyComboScore& r = results[c0 + c];
-            r = SkyComboScore{};
-            r.finite = n;
-            if (n == 0) {
-                r.mean = r.rmse = r.p50 = r.p90 = r.p95 = r.p99 = r.max = r.score = std::nan("");
-                continue;
-            }
-            r.mean = h_sums[c * 3] / double(n);
-            r.rmse = std::sqrt(h_sums[c * 3 + 1] / double(n));
-            for (uint32_t q = 0; q < kTargets; ++q) {  // percentile_sorted: round((n - 1) q), half away from 0
-                tcombo[targets] = c;
-                tprefix[targets] = 0;
-                rank[targets] = uint64_t(std::floor(double(n - 1) * quantiles[q] + 0.5));
-                ++targets;
-            }
+        ScoreLaunch w{};
+        w.bands = bands;
+        w.samples = samples;
+        w.ref_lab = ref_oklab;
+        w.inv_scale = 1.0f / reference_scale;
+        w.combo_bands = reinterpret_cast<const uint32_t*>(base + o_bands) + size_t(c0) * channels;
+        w.combo_xyz = reinterpret_cast<const float*>(base + o_xyz) + size_t(c0) * channels * 3;
+        w.combos = std::min(chunk, combo_count - c0);
+        w.channels = channels;
+        w.dist = reinterpret_cast<float*>(base + o_dist);
+        w.state = reinterpret_cast<ScoreState*>(base + o_state) + c0;
+        w.hist = reinterpret_cast<uint32_t*>(base + o_hist);
+        w.sms = uint32_t(sms);
+        if ((e = launch_score(w, stream))) return cuda_fail(SKY_ERR_LAUNCH, "scoring kernel launch", e);
+    }
+    std::vector<ScoreState> state(combo_count);
+    if ((e = cudaMemcpyAsync(state.data(), base + o_state, state.size() * sizeof(ScoreState), cudaMemcpyDeviceToHost,
+                             stream)) ||
+        (e = cudaStreamSynchronize(stream)))
+        return cuda_fail(SKY_ERR_SYNC, "scoring results", e);
+    for (uint32_t c = 0; c < combo_count; ++c) {
+        const ScoreState& S = state[c];
+        SkyComboScore& r = results[c];
+        r = SkyComboScore{};
+        r.finite = S.count;
+        if (S.count == 0) {
+            r.mean = r.rmse = r.p50 = r.p90 = r.p95 = r.p99 = r.max = r.score = std::nan("");
+            continue;
         }
-        // three radix-selection passes over the bits of the non-negative distances
-        const uint32_t shifts[3] = {21u, 10u, 0u}, widths[3] = {11u, 11u, 10u};
-        for (int pass = 0; pass < 3 && targets > 0; ++pass) {
-            if ((e = cudaMemcpyAsync(d_tcombo, tcombo.data(), targets * 4, cudaMemcpyHostToDevice, stream)) ||
-                (e = cudaMemcpyAsync(d_tprefix, tprefix.data(), targets * 4, cudaMemcpyHostToDevice, stream)) ||
-                (e = cudaMemsetAsync(d_hist, 0, size_t(targets) * kScoreHistBins * 4, stream)))
-                return cuda_fail(SKY_ERR_COPY, "selection upload", e);
-            if ((e = launch_select_hist(dist, samples, d_tcombo, d_tprefix, targets, shifts[pass], widths[pass], d_hist,
-                                        uint32_t(sms), stream)))
-                return cuda_fail(SKY_ERR_LAUNCH, "selection kernel launch", e);
-            if ((e = cudaMemcpyAsync(h_hist.data(), d_hist, size_t(targets) * kScoreHistBins * 4,
-                                     cudaMemcpyDeviceToHost, stream)) ||
-                (e = cudaStreamSynchronize(stream)))
-                return cuda_fail(SKY_ERR_SYNC, "selection histogram", e);
-            const uint32_t bins = 1u << widths[pass];
-            for (uint32_t t = 0; t < targets; ++t) {
-                const uint32_t* h = h_hist.data() + size_t(t) * kScoreHistBins;
-                uint64_t below = 0;
-                uint32_t b = 0;
-                for (; b + 1 < bins && below + h[b] <= rank[t]; ++b) below += h[b];
-                rank[t] -= below;
-                tprefix[t] = (tprefix[t] << widths[pass]) | b;
-            }
-        }
-        for (uint32_t t = 0; t < targets; ++t) {
+        r.mean = S.sum / double(S.count);
+        r.rmse = std::sqrt(S.sum_sq / double(S.count));
+        double* slot[kScoreTargets] = {&r.p50, &r.p90, &r.p95, &r.p99, &r.max};
+        for (uint32_t t = 0; t < kScoreTargets; ++t) {
             float v;
-            std::memcpy(&v, &tprefix[t], 4);
-            SkyComboScore& r = results[c0 + tcombo[t]];
-            double* slot[kTargets] = {&r.p50, &r.p90, &r.p95, &r.p99, &r.max};
-            *slot[t % kTargets] = double(v);
+            std::memcpy(&v, &S.prefix[t], 4);
+            *slot[t] = double(v);
         }
-        for (uint32_t c = 0; c < nc; ++c) {
-            SkyComboScore& r = results[c0 + c];
-            if (r.finite) r.score = r.rmse + 0.25 * r.p95;
-        }
+        r.score = r.rmse + 0.25 * r.p95;
     }
     return SKY_OK;
 }

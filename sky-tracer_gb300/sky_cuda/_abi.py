@@ -200,6 +200,8 @@ _SIGNATURES = {
                                                        ctypes.POINTER(SkyAdjointParams),
                                                        ctypes.POINTER(SkyAdjointGrads), _vp]),
     "sky_cuda_bake_majorants": (ctypes.c_int, [_vp, ctypes.POINTER(SkyAdjointParams), _vp, _vp]),
+    "sky_cuda_score_reference": (ctypes.c_int, [_vp, ctypes.c_uint64, ctypes.POINTER(ctypes.c_double), _vp,
+                                                ctypes.POINTER(ctypes.c_double), _vp]),
     "sky_cuda_score_combos": (ctypes.c_int, [_vp, ctypes.c_uint32, ctypes.c_uint64, _vp, ctypes.c_float,
                                              ctypes.POINTER(ctypes.c_uint32), _fp, ctypes.c_uint32, ctypes.c_uint32,
                                              ctypes.POINTER(SkyComboScore), _vp]),

@@ -45,16 +45,22 @@ def score_combos(bands, ref_xyz: np.ndarray, combo_bands, combo_xyz, scale: floa
         raise ValueError("bands must be a [B, N] float32 CUDA tensor")
     bands = bands.contiguous()
     n = bands.shape[1]
-    ref_xyz = np.asarray(ref_xyz, dtype=np.float64).reshape(n, 3)
-    scale = reference_scale(ref_xyz[:, 1]) if scale is None else float(scale)
-    ref_lab = torch.as_tensor(oklab(ref_xyz / scale).astype(np.float32), device=bands.device).contiguous()
+    # the reference's scale and Oklab on the GPU (reference_scale() and oklab() in FP64)
+    ref = torch.as_tensor(np.ascontiguousarray(ref_xyz, dtype=np.float64).reshape(n, 3), device=bands.device)
+    ref_lab = torch.empty((n, 3), dtype=torch.float32, device=bands.device)
+    st = torch.cuda.current_stream().cuda_stream if stream is None else stream
+    used = ctypes.c_double(0.0)
+    check(lib.sky_cuda_score_reference(ctypes.c_void_p(ref.data_ptr()), n,
+                                       None if scale is None else ctypes.byref(ctypes.c_double(float(scale))),
+                                       ctypes.c_void_p(ref_lab.data_ptr()), ctypes.byref(used),
+                                       ctypes.c_void_p(st)), lib)
+    scale = used.value
     cb = np.ascontiguousarray(combo_bands, dtype=np.uint32)
     cx = np.ascontiguousarray(combo_xyz, dtype=np.float32)
     c, k = cb.shape
     if cx.shape != (c, k, 3):
         raise ValueError("combo_xyz must be [C, K, 3] for combo_bands [C, K]")
     res = (SkyComboScore * c)()
-    st = torch.cuda.current_stream().cuda_stream if stream is None else stream
     check(lib.sky_cuda_score_combos(ctypes.c_void_p(bands.data_ptr()), bands.shape[0], n,
                                     ctypes.c_void_p(ref_lab.data_ptr()), scale,
                                     cb.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32)),
