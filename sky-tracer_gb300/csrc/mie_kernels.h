@@ -27,10 +27,14 @@ struct MieItem {
 // Series terms for size parameter x: x + 4.05 x^(1/3) + 2 (Wiscombe 1980), plus one.
 inline uint32_t mie_terms(double x) { return uint32_t(x + 4.05 * std::cbrt(x) + 2.0) + 1u; }
 
-// Coefficients (one thread per item) then angles (one block per item): adds
-// w (|S1|^2 + |S2|^2) / (2 k^2) of every item to phase_acc[band][bins] (FP64,
-// zeroed by the caller) and writes Q_sca, Q_ext and g per item to q[3 * item].
-cudaError_t launch_mie_bake(const MieItem* items, uint32_t count, uint32_t max_terms, double2* dscratch,
-                            float4* ab, double* q, uint32_t bins, double* phase_acc, cudaStream_t stream);
+// Series recurrences, coefficients and angles of bands x radii items (item of
+// band b and radius r at b * radii + r, radii ascending): adds w (|S1|^2 +
+// |S2|^2) / (2 k^2) of every item to phase_acc[band][bins] (FP64, zeroed by the
+// caller) and writes Q_sca, Q_ext and g per item to q[3 * item].  dscratch holds
+// D_n at doff (dterms + 1 per item), riccati psi_n and chi_n at aoff + item
+// (terms + 1 per item).
+cudaError_t launch_mie_bake(const MieItem* items, uint32_t bands, uint32_t radii, uint32_t max_terms,
+                            double2* dscratch, double2* riccati, float4* ab, double* q, uint32_t bins,
+                            double* phase_acc, uint32_t sms, cudaStream_t stream);
 
 }  // namespace sky

@@ -1418,21 +1418,25 @@ extern "C" int sky_cuda_bake_mie_phase(const SkyMieDistribution* dist, const dou
     }
     if (doff * sizeof(double2) + aoff * sizeof(float4) > (uint64_t(16) << 30))
         return set_error(SKY_ERR_INVALID_CONFIG, "bake too large: more than 16 GB of series scratch");
+    int device = 0, sms = 1;
+    if (cudaGetDevice(&device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "no usable CUDA device");
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     DeviceScratch mem;
     MieItem* d_items = nullptr;
-    double2* d_scr = nullptr;
+    double2 *d_scr = nullptr, *d_ric = nullptr;
     float4* d_ab = nullptr;
     double *d_q = nullptr, *d_acc = nullptr;
     cudaError_t e;
-    if ((e = mem.alloc(&d_items, items.size())) || (e = mem.alloc(&d_scr, doff)) || (e = mem.alloc(&d_ab, aoff)) ||
+    if ((e = mem.alloc(&d_items, items.size())) || (e = mem.alloc(&d_scr, doff)) ||
+        (e = mem.alloc(&d_ric, aoff + items.size())) || (e = mem.alloc(&d_ab, aoff)) ||
         (e = mem.alloc(&d_q, items.size() * 3)) || (e = mem.alloc(&d_acc, size_t(band_count) * phase_bins)))
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "Mie bake scratch allocation", e);
     clear_stale_error();
     if ((e = cudaMemcpy(d_items, items.data(), items.size() * sizeof(MieItem), cudaMemcpyHostToDevice)) ||
         (e = cudaMemset(d_acc, 0, size_t(band_count) * phase_bins * sizeof(double))))
         return cuda_fail(SKY_ERR_COPY, "Mie bake upload", e);
-    if ((e = launch_mie_bake(d_items, uint32_t(items.size()), max_terms, d_scr, d_ab, d_q, phase_bins, d_acc,
-                             nullptr)))
+    if ((e = launch_mie_bake(d_items, band_count, D.r_count, max_terms, d_scr, d_ric, d_ab, d_q, phase_bins, d_acc,
+                             uint32_t(sms), nullptr)))
         return cuda_fail(SKY_ERR_LAUNCH, "Mie bake kernels", e);
     std::vector<double> q(items.size() * 3);
     if ((e = cudaMemcpy(q.data(), d_q, q.size() * sizeof(double), cudaMemcpyDeviceToHost)) ||
