@@ -223,6 +223,8 @@ DevLaunch make_launch(const SkyScene* s, const SkyRenderConfig* c) {
     L.inv_width = 1.0f / float(c->width);
     L.inv_height = 1.0f / float(c->height);
     L.spp_reciprocal = ~uint64_t(0) / c->spp;
+    L.pixels_reciprocal = ~uint32_t(0) / (L.width * L.rows);
+    L.width_reciprocal = ~uint32_t(0) / L.width;
     const float rg = s->dev.ground_radius;
     const float oy = rg + std::max(c->observer_altitude_km, 0.0f);
     const float view_height = std::sqrt(0.0f * 0.0f + oy * oy + 0.0f * 0.0f);

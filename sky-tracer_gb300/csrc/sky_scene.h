@@ -124,6 +124,7 @@ struct DevLaunch {
     float lut_side[3];
     float inv_width, inv_height;
     uint64_t spp_reciprocal;  // floor((2^64 - 1) / spp)
+    uint32_t pixels_reciprocal, width_reciprocal;  // floor((2^32 - 1) / (width rows)), / width)
 };
 
 // One render inside a persistent launch: its scene (tables may be shared

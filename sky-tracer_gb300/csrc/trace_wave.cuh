@@ -23,15 +23,17 @@
 //
 // What bounds it: instruction issue.  HBM and the tensor cores have no part in
 // it (16 B leave the chip per cell, and a path is a chain of branches).  The
-// kernel before this one kept each lane's path in registers and ran all event
+// ray loop (trace_ray.cuh) keeps each lane's path in registers and runs all event
 // code once per ray: 9.5 of 32 lanes active per instruction, 7.9 G warp
 // instructions and 7.42 ms for 42 M chains (128x64, 81 bands, 64 spp).  Here
-// 21.5 lanes are active, for 5.0 G instructions and 5.15 ms; what is left is
-// the rays' different lengths, the queues (about 60 instructions to take a
-// batch and 60 to put it back, for some 800 that work on it) and instruction
-// fetch (a third of the stalls: the stages are large, and a scheduler's warps
-// are in different ones).  Tracking right after the stage, instead of queueing
-// every ray for it, took 6.2 to 5.4 ms, staying with a stage 5.4 to 5.15.
+// 21 lanes are active, for 5.1 G instructions at 87 % of the issue slots and 4.65
+// ms; what is left is the rays' different lengths (tracking is two fifths) and
+// the queues (a fifth).  What took it there: tracking right after the stage,
+// instead of queueing every ray for it, 6.2 to 5.4 ms; staying with a stage, 5.15
+// (instruction fetch was the first stall: the stages are large, and a scheduler's
+// warps are in different ones); one copy of the rays' set-up for all stages,
+// 4.87; products for the start's quotients, 4.84; the tracking loop's crossings
+// and parking limits, 4.65.
 //
 // Each chain consumes its random stream in the plain kernel's order
 // (trace_path, sky_trace.wgsl:703-776), so both kernels trace the same paths.
@@ -58,10 +60,15 @@ constexpr uint32_t kMaxIdlePolls = 1u << 30;   // polls of empty queues (>= 100 
 constexpr uint32_t kMaxSlotPolls = 1u << 24;   // polls of one queue slot before the same
 
 // Rays still under way when a warp leaves the tracking loop and puts them back:
-// most of a warp's rays end within a few steps, a few take many times that.
-// Merged layers: 4 to 16 measured within 1 % of each other (128x64, 81 bands, 64
-// spp); the other modes, layer by layer: 8 is 6 % slower than 12, 16 the same.
-constexpr uint32_t kPark = 8, kParkLayered = 12;
+// most of a warp's rays end within a few steps, a few take many times that.  The
+// fewer steps a queue entry costs, the more are left: merged layers (2.3 steps a
+// ray) 8 -> 14 of 32 takes 4.74 to 4.65 ms (128x64, 81 bands, 64 spp), 20 4.68;
+// the other modes, layer by layer (some 30 steps), 12 -> 26 takes 6.06 to 4.85 ms
+// (64x32, 41 bands, 64 spp), 28 the same.
+constexpr uint32_t kPark = 14, kParkLayered = 26;
+// Rays that still have a crossing to make when a warp turns to its tentative
+// collisions.
+constexpr uint32_t kCrossing = 3;
 
 
 // Blocks per SM.  A kernel shape is the warps of a block (SkyTuning.variant).
@@ -137,6 +144,17 @@ __device__ __forceinline__ Rng path_rng(const float4& C, uint32_t dim) {
     return r;
 }
 
+// a / d and its remainder, from floor((2^32 - 1) / d).
+__device__ __forceinline__ uint32_t quotient(uint32_t a, uint32_t d, uint32_t reciprocal, uint32_t& rest) {
+    uint32_t q = __umulhi(a, reciprocal);
+    rest = a - q * d;
+    if (rest >= d) {
+        ++q;
+        rest -= d;
+    }
+    return q;
+}
+
 // Start of a ray's tracking: what of the tracker's state depends on the ray
 // alone, and the first draws.  Fills B and the layer bits of C.z.
 template <int kTracking>
@@ -167,8 +185,8 @@ __device__ __forceinline__ uint32_t track_batch(const DevScene& S, const Medium&
     float t = B.x;
     uint32_t ended = 0u;
     if constexpr (kTracking == SKY_TRACKING_MERGED_LAYERS) {
-        // track_ray_merged: a step is one crossing at most, then one tentative collision
-        // at most (two crossings a step: +1 %)
+        // track_ray_merged: a step is the ray's crossings up to the segment that holds its
+        // next tentative collision (or some of them), then that collision
         const MergedGrid G = merged_grid(S, band);
         int m = int((meta >> 16) & 0xfffu), dir = int(meta >> 28) - 1;
         float tau = B.y, t_seg = B.z;
@@ -177,9 +195,9 @@ __device__ __forceinline__ uint32_t track_batch(const DevScene& S, const Medium&
             // the next tentative collision: one expression, which the compiler contracts into
             // the multiply-add that the plain kernel rounds with
             float next_t = 0.0f;
-            if (alive) {
-                next_t = t + tau / maj;
-                if (!(next_t < t_seg)) {
+            if (alive) next_t = t + tau / maj;
+            for (;;) {  // the crossings, until few rays have more to make (one each: +1.5 %)
+                if (alive && !(next_t < t_seg)) {
                     if (dir == 0) {
                         ended = kMiss;
                         alive = false;
@@ -193,6 +211,7 @@ __device__ __forceinline__ uint32_t track_batch(const DevScene& S, const Medium&
                         next_t = t + tau / maj;
                     }
                 }
+                if (__popc(__ballot_sync(kFull, alive && !(next_t < t_seg))) <= kCrossing) break;
             }
             if (alive && next_t < t_seg) {
                 t = next_t;
@@ -290,30 +309,6 @@ __device__ __forceinline__ uint32_t track_batch(const DevScene& S, const Medium&
     return ended;
 }
 
-// The outgoing ray of a vertex or camera (sky_trace.wgsl:709-717): false when
-// the chain ends here.
-template <int kTracking>
-__device__ __forceinline__ bool primary_ray(const DevScene& S, const DevLaunch& JL, V3 org, V3 dir, uint32_t depth,
-                                            uint32_t band, Rng& rng, float& rad, float4& A, float4& B, uint32_t& meta,
-                                            Counters& n, bool& watchdog) {
-    if (depth >= JL.watchdog_limit) {
-        watchdog = true;
-        return false;
-    }
-    const RayGeo g = ray_geo(org, dir);
-    ++n.e[SKY_EVENT_BOUNDARY];
-    float t_max;
-    uint32_t boundary;
-    if ((JL.max_orders != 0u && depth >= JL.max_orders) || !next_boundary(S, g, t_max, boundary)) {
-        rad = fmaxf(rad, 0.0f);
-        return false;
-    }
-    meta = band | (boundary == 1u ? uint32_t(kFlagTop) : 0u);
-    track_begin<kTracking>(S, g, t_max, band, rng, B, meta, n);
-    A = make_float4(g.b, g.p, g.r0sq, t_max);
-    return true;
-}
-
 // kCount: count events (SkyDeviceOutputs.counters given).  Without it the
 // counters are never read, so their increments compile away.
 // kAer: aerosol species evaluated by the medium functions (1 or kSpecies,
@@ -323,7 +318,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     wave_kernel(const __grid_constant__ DevScene S, const __grid_constant__ DevLaunch L0,
                 const DevJob* __restrict__ jobs, uint32_t num_jobs, unsigned long long total_chains, uint32_t paths,
                 uint32_t used_paths, unsigned long long* __restrict__ work_counter,
-                unsigned long long* __restrict__ counters, uint32_t* __restrict__ status, uint64_t batch_limit) {
+                unsigned long long* __restrict__ counters, uint32_t* __restrict__ status, uint32_t batch_limit) {
     constexpr uint32_t kRows = path_rows<kAer>();
     extern __shared__ __align__(16) unsigned char smem[];
     float4* const pool = reinterpret_cast<float4*>(smem + pool_offset(S.knot_count, S.band_count));
@@ -347,7 +342,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     bool watchdog = false;
     uint32_t idle = 0u, turn = (threadIdx.x >> 5) & 3u;
 
-    for (uint64_t batch = 0u;;) {
+    for (uint32_t batch = 0u;;) {
         // the fullest queue: lanes 0-3 look at one each.  A lane's head, read before its
         // tail, goes with its own count: the exchange below fails if the head has moved
         // since, so what it takes has been put there.
@@ -406,8 +401,9 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
         fence_block();
         float4* const P = pool + id * kRows;
         uint32_t next = kQNone;
-        // the lane's ray: set up by its stage, or taken up where it was left
-        bool tracing = false;
+        // the lane's ray: set up from its stage's origin and direction, or taken up where it was left
+        bool tracing = false, set_up = false;
+        V3 ray_org = mk(0.0f, 0.0f, 0.0f), ray_dir = ray_org;
         float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = A;
         uint32_t meta = 0u;
         Rng rng;
@@ -468,10 +464,9 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
                     // (:587-608), one shadow ray at a time
                     rng = path_rng(C, as_u(B.w));
                     const uint32_t lights = JL.direct_light_samples;
-                    bool lit = false;
                     meta = band | kFlagShadow | (ground ? uint32_t(kFlagGround) : 0u);
-                    RayGeo g;
-                    float t_max = 0.0f, nee_mu = 0.0f;
+                    next = kQContinue;
+                    B = make_float4(0.0f, as_f(kHit), 0.0f, 0.0f);  // no sun: as a shadow ray that collides
                     while (ls < lights) {
                         ++ls;
                         const V3 ldir = sample_sun_cone(job_scene<kSingle>(S, jobs, job), rng);
@@ -481,25 +476,15 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
                             cos_sun = fmaxf(dot3(normalize_or_y(org), ldir), 0.0f);
                             if (!(cos_sun > 0.0f)) continue;
                         }
-                        g = ray_geo(madd(org, ldir, kRayEpsilonKm), ldir);
-                        uint32_t kind;
-                        ++n.e[SKY_EVENT_BOUNDARY];
-                        if (!(next_boundary(S, g, t_max, kind) && kind == 1u)) continue;
-                        nee_mu = ground ? cos_sun : dot3(dir, ldir);
-                        lit = true;
+                        ray_org = madd(org, ldir, kRayEpsilonKm);
+                        ray_dir = ldir;
+                        reinterpret_cast<float*>(&P[kF])[3] = ground ? cos_sun : dot3(dir, ldir);
+                        set_up = true;
                         break;
                     }
-                    if (lit) {
-                        track_begin<kTracking>(S, g, t_max, band, rng, B, meta, n);
-                        A = make_float4(g.b, g.p, g.r0sq, t_max);
-                        reinterpret_cast<float*>(&P[kF])[3] = nee_mu;
-                        tracing = true;
-                    } else {
-                        // no sun: as a shadow ray that collides
-                        P[kB] = make_float4(0.0f, as_f(kHit), 0.0f, as_f(rng.dim));
-                        reinterpret_cast<float*>(&P[kC])[2] = as_f(meta);
-                        next = kQContinue;
-                    }
+                    B.w = as_f(rng.dim);
+                    P[kB] = B;
+                    reinterpret_cast<float*>(&P[kC])[2] = as_f(meta);
                     reinterpret_cast<float*>(&P[kC])[3] = as_f(job | (ls << 16));
                 }
             }
@@ -603,15 +588,19 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
                             ++depth;
                         }
                     }
-                    if (alive)
-                        alive = primary_ray<kTracking>(S, JL, org, dir, depth, band, rng, rad, A, B, meta, n, watchdog);
-                    if (alive) {
-                        P[kD] = make_float4(org.x, org.y, org.z, thr);
-                        P[kE] = make_float4(dir.x, dir.y, dir.z, rad);
-                        reinterpret_cast<float*>(&P[kF])[0] = as_f(depth);
-                        tracing = true;
-                    } else {
-                        reinterpret_cast<float*>(&P[kE])[3] = rad;
+                    if (alive && depth >= JL.watchdog_limit) {
+                        watchdog = true;
+                        alive = false;
+                    }
+                    // what the next ray finds at its boundary may still end the chain, with this radiance
+                    P[kD] = make_float4(org.x, org.y, org.z, thr);
+                    P[kE] = make_float4(dir.x, dir.y, dir.z, rad);
+                    reinterpret_cast<float*>(&P[kF])[0] = as_f(depth);
+                    set_up = alive;
+                    ray_org = org;
+                    ray_dir = dir;
+                    meta = band;
+                    if (!alive) {
                         reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
                         next = kQStart;
                     }
@@ -655,33 +644,29 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
                 }
                 const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
                 const unsigned long long rel = kSingle ? at : at - __ldg(&jobs[job].chain_begin);
-                // rel / spp: the product with floor((2^64 - 1) / spp) is at most one short
+                // cell and sample, band and pixel of the slab, row and column: quotients by products
+                // with floor((2^k - 1) / divisor), which are at most one short
                 uint32_t c = uint32_t(__umul64hi(rel, JL.spp_reciprocal));
                 uint32_t sample = uint32_t(rel - (unsigned long long)c * JL.spp);
                 if (sample >= JL.spp) {
                     ++c;
                     sample -= JL.spp;
                 }
-                const uint32_t npix = JL.width * JL.rows;
-                const uint32_t band = c / npix;
-                const uint32_t slab_pixel = c - band * npix;
-                const uint32_t row = slab_pixel / JL.width;  // row within the job's slab
-                const uint32_t px = slab_pixel - row * JL.width, py = row + JL.row_begin;
+                uint32_t slab_pixel, px;
+                const uint32_t band = quotient(c, JL.width * JL.rows, JL.pixels_reciprocal, slab_pixel);
+                const uint32_t py = quotient(slab_pixel, JL.width, JL.width_reciprocal, px) + JL.row_begin;
                 // the image pixel drives the random stream, the slab pixel indexes the sums
                 rng.init(py * JL.width + px, JL.sample_offset + sample, band, JL.seed_lo, JL.seed_hi);
                 const V3 dir = camera_dir(JL, px, py, rng);
                 const V3 org = mk(0.0f, S.ground_radius + fmaxf(JL.observer_altitude, 0.0f), 0.0f);
                 ++n.e[SKY_EVENT_CHAIN];
-                float new_rad = 0.0f;
                 meta = band;
-                tracing = primary_ray<kTracking>(S, JL, org, dir, 0u, band, rng, new_rad, A, B, meta, n, watchdog);
-                if (!tracing) {
-                    reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
-                    next = kQStart;
-                }
-                P[kC] = make_float4(as_f(rng.k0), as_f(rng.k1), as_f(meta), as_f(job));
+                set_up = true;
+                ray_org = org;
+                ray_dir = dir;
+                P[kC] = make_float4(as_f(rng.k0), as_f(rng.k1), as_f(band), as_f(job));
                 P[kD] = make_float4(org.x, org.y, org.z, 1.0f);
-                P[kE] = make_float4(dir.x, dir.y, dir.z, new_rad);
+                P[kE] = make_float4(dir.x, dir.y, dir.z, 0.0f);
                 P[kF] = make_float4(as_f(0u), as_f(slab_pixel * S.band_count + band), 0.0f, 0.0f);
             }
             const uint32_t gone = __popc(__ballot_sync(kFull, on && !more));
@@ -695,12 +680,46 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
             }
         }
 
+        // the stages' rays: a shadow ray goes to the sun or leaves its vertex without one
+        // (sky_trace.wgsl:574-577), an outgoing ray ends the chain where it meets no boundary
+        // (:709-717).  One copy of this code for all stages: it is a third of theirs, and the
+        // instruction caches are short of room.
+        if (set_up) {
+            const RayGeo g = ray_geo(ray_org, ray_dir);
+            const bool shadow = (meta & kFlagShadow) != 0u;
+            const uint32_t word = as_u(reinterpret_cast<const float*>(&P[kC])[3]);
+            const DevLaunch& JL = job_launch<kSingle>(L0, jobs, word & 0xffffu);
+            ++n.e[SKY_EVENT_BOUNDARY];
+            float t_max;
+            uint32_t boundary;
+            bool ok = next_boundary(S, g, t_max, boundary);
+            if (shadow) {
+                ok = ok && boundary == 1u;
+                if (!ok && (word >> 16) < JL.direct_light_samples) next = kQVertex;  // the next sample
+            } else {
+                const uint32_t max_orders = JL.max_orders;
+                if (max_orders != 0u && as_u(reinterpret_cast<const float*>(&P[kF])[0]) >= max_orders) ok = false;
+                if (boundary == 1u) meta |= kFlagTop;
+                if (!ok) {
+                    float* rad = reinterpret_cast<float*>(&P[kE]) + 3;
+                    *rad = fmaxf(*rad, 0.0f);
+                    reinterpret_cast<float*>(&P[kB])[1] = as_f(kOver);
+                    next = kQStart;
+                }
+            }
+            if (ok) {
+                track_begin<kTracking>(S, g, t_max, meta & 255u, rng, B, meta, n);
+                A = make_float4(g.b, g.p, g.r0sq, t_max);
+                tracing = true;
+            }
+        }
         // track the rays at once, whatever stage they come from
         const uint32_t rays = __popc(__ballot_sync(kFull, tracing));
         if (rays) {
             const RayGeo g{A.x, A.y, A.z};
-            // park few rays, and fewer of a small batch
-            const uint32_t park = min(kTracking == SKY_TRACKING_MERGED_LAYERS ? kPark : kParkLayered, rays * 3u / 8u);
+            // fewer of a small batch
+            const uint32_t park = kTracking == SKY_TRACKING_MERGED_LAYERS ? min(kPark, rays / 2u)
+                                                                          : min(kParkLayered, rays * 7u / 8u);
             const uint32_t ended = track_batch<kTracking>(S, M, tracing, g, A.w, meta & 255u,
                                                           (meta & kFlagShadow) != 0u, rng, B, meta, n, watchdog, park);
             if (tracing) {
@@ -789,7 +808,8 @@ cudaError_t launch_wave_shape(const WaveLaunch& w, cudaStream_t stream) {
     const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * sms, want)));
     const uint64_t share = ((w.total_chains + blocks - 1u) / blocks + 31u) / 32u * 32u;
     const uint32_t used = uint32_t(std::min<uint64_t>(paths, share));
-    const uint64_t limit = uint64_t(w.iteration_limit ? w.iteration_limit : kMaxIterations) * kBatchesPerIteration;
+    const uint32_t limit = uint32_t(std::min<uint64_t>(
+        0xffffffffu, uint64_t(w.iteration_limit ? w.iteration_limit : kMaxIterations) * kBatchesPerIteration));
     wave_kernel<kTracking, kPhase, kWarps, kSingle, kCount, kAer><<<blocks, kThreads, smem, stream>>>(
         w.scene, w.launch0, w.jobs, w.num_jobs, w.total_chains, paths, used, w.work_counter, w.counters, w.status,
         limit);
