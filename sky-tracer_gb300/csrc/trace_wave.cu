@@ -31,17 +31,18 @@ __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restr
 // queues (trace_wave.cuh): where it has so few chains per lane of the chip
 // (1024 lanes per SM) that its longest chains decide its time.  Measured with
 // both kernels (ms, ray loop against queues):
-//   merged layers      3.1 M chains 0.63 / 0.68, 5.2 M 0.97 / 0.90 (one species);
-//                      4.0 M 1.46 / 1.51, 6.7 M 2.12 / 1.77 (four): 28 per lane
-//   residual carry     1.3 M 1.34 / 1.37, 2.1 M 1.94 / 1.89: 10 per lane
-//   segment restart    0.67 M 1.26 / 1.43, 1.0 M 1.64 / 1.28: 6 per lane
+//   merged layers      one species: 3.1 M chains 0.63 / 0.65, 4.2 M 0.79 / 0.75: 24 per lane;
+//                      four: 4.0 M 1.47 / 1.60, 5.4 M 1.86 / 1.81: 34 per lane
+//   residual carry     131 k 0.52 / 0.68, 262 k 0.63 / 0.62, 524 k 0.82 / 0.70: 2 per lane
+//   segment restart    0.67 M 1.25 / 1.34, 1.0 M 1.63 / 1.12: 5 per lane
 cudaError_t small_render(const WaveLaunch& w, bool& small) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t per_lane = w.tracking == SKY_TRACKING_SEGMENT_RESTART  ? 6u
-                              : w.tracking == SKY_TRACKING_RESIDUAL_CARRY ? 10u
-                                                                          : 28u;
+    const uint64_t per_lane = w.tracking == SKY_TRACKING_SEGMENT_RESTART  ? 5u
+                              : w.tracking == SKY_TRACKING_RESIDUAL_CARRY ? 2u
+                              : w.aerosol_species == 1u                   ? 24u
+                                                                          : 34u;
     small = w.total_chains < per_lane * 1024u * uint64_t(sms);
     return e;
 }

@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 MERGED, CARRY, RESTART = _abi.TRACKING_MERGED_LAYERS, _abi.TRACKING_RESIDUAL_CARRY, _abi.TRACKING_SEGMENT_RESTART
 # chains per lane from which a mode takes the queues
-PER_LANE = {MERGED: 28, CARRY: 10, RESTART: 6}
+PER_LANE = {MERGED: 34, CARRY: 2, RESTART: 5}
 
 
 def _samples(cells: int, tracking: int) -> int:
