@@ -68,6 +68,7 @@ struct AdjJob {
     float* chain_rad;
     uint32_t cell_begin;  // first global cell of the render in the launch
     uint32_t cell_count;
+    uint64_t chain_begin; // first chain of the render in the launch (cells times samples)
 };
 
 // The renders of one launch, passed by value as a kernel parameter (no job
@@ -77,6 +78,7 @@ struct AdjJobs {
     AdjJob j[kAdjMaxJobs];
     uint32_t count;
     uint32_t cells;  // sum of the renders' cells
+    uint64_t chains; // sum over the renders of cells times samples
 };
 
 // Writable views of the tables the prepare kernel fills.
@@ -88,7 +90,7 @@ struct AdjWorkspace {
     float* maj;
     uint16_t* map;
     uint32_t* count;
-    uint32_t* next_cell;  // work counter of the adjoint kernel
+    unsigned long long* next_cell;  // work counter of the adjoint kernels
 };
 
 // Scene workspace layout for a scene of B bands, L layers and `bins` phase bins.
@@ -105,13 +107,20 @@ cudaError_t launch_adjoint_prepare(const AdjCtx& A, const AdjWorkspace& W, cudaS
 // A batch (J) takes the ray loop and needs P = Q; the warp-per-cell form
 // renders J.j[0] alone.
 cudaError_t launch_adjoint_primal(const AdjCtx& A, const AdjJobs& J, bool accumulate, unsigned long long* counters,
-                                  uint32_t* status, uint32_t* next_cell, cudaStream_t stream);
+                                  uint32_t* status, unsigned long long* next_cell, cudaStream_t stream);
 
 // Path-replay gradient (P == Q): adds dLoss/dparams to layer_grad [3 L + 2]
 // and band_grad [B][4] (may be null) given each render's dLoss/dfilm
 // [pixels][B] (J.j[i].dloss).
 cudaError_t launch_adjoint_grad(const AdjCtx& A, const AdjJobs& J, double* layer_grad, double* band_grad,
-                                unsigned long long* counters, uint32_t* status, uint32_t* next_cell,
+                                unsigned long long* counters, uint32_t* status, unsigned long long* next_cell,
                                 cudaStream_t stream);
+
+// Whether a launch is small for the stage queues (adjoint_wave.cu), and the
+// queue kernels themselves: the primal (grad = false) over P = Q, adding into the
+// cell sums, and the path-replay gradient with segment integrals.  No counters.
+cudaError_t adjoint_small(const AdjJobs& J, bool grad, bool& small);
+cudaError_t launch_adjoint_wave(const AdjCtx& A, const AdjJobs& J, bool grad, double* layer_grad, double* band_grad,
+                                uint32_t* status, unsigned long long* work_counter, cudaStream_t stream);
 
 }  // namespace sky

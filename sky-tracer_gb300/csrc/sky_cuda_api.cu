@@ -1001,8 +1001,10 @@ int adjoint_place(AdjJobs& J, AdjJob& job) {
     if (uint64_t(J.cells) + job.cell_count > kMaxLaunchCells)
         return set_error(SKY_ERR_INVALID_CONFIG, "a launch holds at most 4026531840 (pixel, band) cells");
     job.cell_begin = J.cells;
+    job.chain_begin = J.chains;
     J.j[J.count++] = job;
     J.cells += job.cell_count;
+    J.chains += uint64_t(job.cell_count) * job.L.spp;
     return SKY_OK;
 }
 

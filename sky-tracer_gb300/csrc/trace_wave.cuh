@@ -48,6 +48,7 @@
 
 #include <algorithm>
 
+#include "stage_queues.cuh"
 #include "trace_common.cuh"
 
 namespace sky {
@@ -56,8 +57,6 @@ namespace wave {
 // Batches of a warp that count as one iteration of SkyTuning.iteration_limit (32
 // chains take about 3.7 batches and 3 rays).
 constexpr uint64_t kBatchesPerIteration = 4;
-constexpr uint32_t kMaxIdlePolls = 1u << 30;   // polls of empty queues (>= 100 ns each) before the same
-constexpr uint32_t kMaxSlotPolls = 1u << 24;   // polls of one queue slot before the same
 
 // Rays still under way when a warp leaves the tracking loop and puts them back:
 // most of a warp's rays end within a few steps, a few take many times that.  The
@@ -73,8 +72,6 @@ constexpr uint32_t kCrossing = 3;
 
 // Blocks per SM.  A kernel shape is the warps of a block (SkyTuning.variant).
 constexpr int kBlocksPerSm = 2;
-
-enum : uint32_t { kQTrack = 0u, kQVertex = 1u, kQContinue = 2u, kQStart = 3u, kQueues = 4u, kQNone = 7u };
 
 // How a ray ended (Path B.y): a real collision at t, the boundary, or no ray
 // at all (the chain's radiance is final; the path has no chain yet).
@@ -100,24 +97,6 @@ __host__ __device__ constexpr uint32_t path_rows() {
     return kAer == 1 ? 7u : 9u;
 }
 
-// The stage queues of a block: rings of path numbers with counters of what was
-// ever taken (head) and put (tail).  A slot holds kEmpty unless a path number
-// is waiting in it.
-constexpr uint32_t kEmpty = 0xffffu;
-struct Queues {
-    uint32_t head[kQueues];
-    uint32_t tail[kQueues];
-    uint32_t live;   // paths that may still have work
-    uint32_t _pad[3];
-};
-
-__host__ __device__ inline uint32_t queue_slots(uint32_t paths) {
-    uint32_t n = 32u;
-    while (n < paths) n <<= 1;
-    return n;
-}
-
-__host__ __device__ inline size_t align16(size_t v) { return (v + 15u) & ~size_t(15u); }
 __host__ __device__ inline size_t pool_offset(uint32_t knots, uint32_t bands) {
     return align16(staged_medium_bytes(knots, bands));
 }
@@ -127,13 +106,6 @@ __host__ __device__ inline size_t wave_smem_bytes(uint32_t knots, uint32_t bands
     return pool_offset(knots, bands) + size_t(paths) * path_rows<kAer>() * 16u + sizeof(Queues) +
            size_t(kQueues) * queue_slots(paths) * sizeof(uint16_t);
 }
-
-// Orders a warp's accesses to paths before (after) it puts them into (takes
-// them from) a queue.
-__device__ __forceinline__ void fence_block() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
-
-__device__ __forceinline__ float as_f(uint32_t v) { return __uint_as_float(v); }
-__device__ __forceinline__ uint32_t as_u(float v) { return __float_as_uint(v); }
 
 __device__ __forceinline__ Rng path_rng(const float4& C, uint32_t dim) {
     Rng r;
@@ -323,19 +295,10 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     extern __shared__ __align__(16) unsigned char smem[];
     float4* const pool = reinterpret_cast<float4*>(smem + pool_offset(S.knot_count, S.band_count));
     Queues* const Q = reinterpret_cast<Queues*>(pool + size_t(paths) * kRows);
-    volatile uint16_t* const slots = reinterpret_cast<volatile uint16_t*>(Q + 1);
-    const uint32_t ring = queue_slots(paths), mask = ring - 1u;
+    const StageQueues queues(Q, paths, used_paths);
     const uint32_t lane = threadIdx.x & 31u;
-    // every path starts without a chain, in the start queue
-    for (uint32_t i = threadIdx.x; i < kQueues * ring; i += blockDim.x)
-        slots[i] = uint16_t(i >= kQStart * ring && i < kQStart * ring + used_paths ? i - kQStart * ring : kEmpty);
     for (uint32_t i = threadIdx.x; i < used_paths; i += blockDim.x)
         pool[i * kRows + kB] = make_float4(0.0f, as_f(kFresh), 0.0f, 0.0f);
-    if (threadIdx.x < kQueues) {
-        Q->head[threadIdx.x] = 0u;
-        Q->tail[threadIdx.x] = threadIdx.x == kQStart ? used_paths : 0u;
-    }
-    if (threadIdx.x == 0u) Q->live = used_paths;
     const Medium M = stage_medium(S, smem);  // ends with the block's only barrier
     Counters n;
     n.clear();
@@ -343,62 +306,11 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     uint32_t idle = 0u, turn = (threadIdx.x >> 5) & 3u;
 
     for (uint32_t batch = 0u;;) {
-        // the fullest queue: lanes 0-3 look at one each.  A lane's head, read before its
-        // tail, goes with its own count: the exchange below fails if the head has moved
-        // since, so what it takes has been put there.
-        uint32_t h = 0u, count = 0u;
-        if (lane < kQueues) {
-            h = *reinterpret_cast<volatile uint32_t*>(&Q->head[lane]);
-            count = *reinterpret_cast<volatile uint32_t*>(&Q->tail[lane]) - h;
-        }
-        // a full batch if there is one, of the warp's last stage rather than of another:
-        // warps that stay with a stage keep its code in the instruction caches (fullest
-        // queue first: +8 %, stages in turn: +4 %); else the fullest queue
-        const uint32_t full = __ballot_sync(kFull, count >= 32u);
-        uint32_t stage, waiting = 32u;
-        if (full) {
-            stage = (uint32_t(__ffs(int((full | (full << 4)) >> turn))) - 1u + turn) & 3u;
-            turn = stage;
-        } else {
-            const uint32_t best = __reduce_max_sync(kFull, (count << 2) | (lane & 3u));
-            stage = best & 3u;
-            waiting = best >> 2;
-        }
-        if (waiting == 0u) {
-            // one lane looks for all: the warp leaves together
-            if (__shfl_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&Q->live), 0) == 0u) break;
-            if (++idle >= kMaxIdlePolls) {
-                if (lane == 0u) atomicOr(status, 2u);
-                break;
-            }
-            __nanosleep(100);
-            __syncwarp();
-            continue;
-        }
-        if (batch >= batch_limit) {  // warp-uniform
-            if (lane == 0u) atomicOr(status, 2u);
-            break;
-        }
-        const uint32_t take = min(waiting, 32u);
-        h = __shfl_sync(kFull, h, stage);
-        uint32_t seen = 0u;
-        if (lane == 0u) seen = atomicCAS(&Q->head[stage], h, h + take);
-        if (__shfl_sync(kFull, seen, 0) != h) continue;  // another warp was first
-        ++batch;
+        uint32_t stage, take, id;
+        const Taken taken = queues.take(lane, turn, idle, batch, batch_limit, status, stage, take, id);
+        if (taken == kOutOfWork) break;
+        if (taken == kNothing) continue;
         const bool on = lane < take;
-        uint32_t id = 0u;
-        if (on) {
-            volatile uint16_t* slot = slots + stage * ring + ((h + lane) & mask);
-            uint32_t v = *slot, polls = 0u;
-            while (v == kEmpty && ++polls < kMaxSlotPolls) v = *slot;  // put, but not yet written
-            *slot = uint16_t(kEmpty);
-            id = v;
-            if (v == kEmpty) {
-                atomicOr(status, 2u);
-                id = 0u;
-            }
-        }
-        fence_block();
         float4* const P = pool + id * kRows;
         uint32_t next = kQNone;
         // the lane's ray: set up from its stage's origin and direction, or taken up where it was left
@@ -732,23 +644,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
             }
         }
 
-        // each path into the queue of its next stage: one lane of those that go to a queue
-        // takes room for all of them
-        const uint32_t own = __match_any_sync(kFull, next);
-        const uint32_t first = uint32_t(__ffs(int(own))) - 1u;
-        fence_block();
-        uint32_t room = 0u;
-        if (lane == first && next != kQNone) room = atomicAdd(&Q->tail[next], uint32_t(__popc(own)));
-        room = __shfl_sync(kFull, room, first);
-        if (next != kQNone) {
-            volatile uint16_t* slot =
-                slots + next * ring + ((room + __popc(own & ((1u << lane) - 1u))) & mask);
-            uint32_t polls = 0u;
-            while (*slot != kEmpty && ++polls < kMaxSlotPolls) {}  // its last path is being taken
-            if (polls >= kMaxSlotPolls) atomicOr(status, 2u);
-            *slot = uint16_t(id);
-        }
-        __syncwarp();
+        queues.put(lane, next, id, status);
     }
     if (kCount) {
 #pragma unroll
