@@ -15,10 +15,12 @@
 //
 // What bounds it: instruction issue, as the tracer.  The ray loop runs all event
 // code once per ray: 8 to 10 of 32 lanes active.  16.8 M chains (128x64, 32 bands,
-// 64 spp): primal 3.79 -> 2.20 ms, gradient with the primal's chain radiance 4.05 ->
-// 3.44 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.2 ms and
-// 29.7 -> 21.2 ms.  The gradient is still short of instructions (46 % of the issue
-// slots, no instruction the first stall): its code is more than the caches hold.
+// 64 spp): primal 3.79 -> 2.18 ms, gradient with the primal's chain radiance 4.05 ->
+// 3.09 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.1 ms and
+// 29.7 -> 20.2 ms.  The primal issues at 83 % with 24 lanes active; the gradient at
+// 52 % with 17: its code is still more than the instruction caches hold ("no
+// instruction" 3.0 cycles per issue), and its layer gradients are shared-memory
+// atomics (short scoreboard 2.3).
 
 #include <algorithm>
 
@@ -58,9 +60,8 @@ constexpr uint32_t kPark = 14, kCrossing = 3;
 // A path in shared memory, rows of 16 bytes: A-F as the tracer's, then
 //   G  the vertex: unscaled Rayleigh, Mie and ozone coefficients, layer
 //   H  (gradient) majorant optical depth and start of the ray's current piece,
-//      the chain's radiance, the weight of a sun sample's term
-//   I  (gradient) loss weight, the sun sample's term, the random stream's
-//      position at the ray's start
+//      the chain's radiance
+//   I  (gradient) loss weight; the random stream's position at the ray's start
 enum : uint32_t { kA = 0u, kB = 1u, kC = 2u, kD = 3u, kE = 4u, kF = 5u, kG = 6u, kH = 7u, kI = 8u };
 template <bool kGrad>
 __host__ __device__ constexpr uint32_t path_rows() {
@@ -164,14 +165,41 @@ __device__ __forceinline__ float mixed(const AdjMed& m, float rayleigh, float mi
     const float r = __fmul_rn(m.R, rayleigh);
     return m.Ms > 0.0f ? __fmaf_rn(m.Ms, mie, r) : r;
 }
-__device__ __forceinline__ float mixed_phase_value(const AdjSet& X, uint32_t bins, const AdjMed& m, float mu) {
-    return mixed(m, rayleigh_phase(mu), m.Ms > 0.0f ? hg_value(X, bins, mu) : 0.0f);
-}
-// The NEE term's phase, normalised by the scattering coefficient.
-__device__ __forceinline__ float nee_phase(const AdjSet& X, uint32_t bins, const AdjMed& m, float mu) {
-    if (!(m.s > 0.0f)) return 0.0f;
-    const float mie = m.Ms > 0.0f ? __fmul_rn(m.Ms, hg_value(X, bins, mu)) : 0.0f;
-    return __fadd_rn(__fmul_rn(m.R, rayleigh_phase(mu)), mie) / m.s;
+// The HG table at a cosine: hg_value() and the terms of vertex_terms().
+struct HgSlot {
+    float p0, p1, d0, d1, t;
+    __device__ __forceinline__ HgSlot(const AdjSet& X, uint32_t bins, float mu) {
+        uint32_t i0, i1;
+        hg_slot(bins, mu, i0, i1, t);
+        p0 = __ldg(X.phase + i0);
+        p1 = __ldg(X.phase + i1);
+        d0 = __ldg(X.dphase + i0);
+        d1 = __ldg(X.dphase + i1);
+    }
+    __device__ __forceinline__ float value() const { return fmaxf(fmaf(t, p1 - p0, p0), 0.0f); }
+    __device__ __forceinline__ float slope() const { return fmaf(t, d1 - d0, d0); }
+};
+
+// vertex_terms() with the table's values at hand.
+__device__ __forceinline__ void vertex_terms_at(AdjAcc& a, const AdjSet& X, const HgSlot& slot, const AdjBase& b,
+                                                const AdjMed& m, float pr, float weight) {
+    if (weight == 0.0f) return;
+    const float pm = slot.value();
+    const float sum = m.R * pr + m.Ms * pm;
+    if (!(sum > 0.0f)) return;
+    const float w = weight / sum;
+    const float* p = X.layer + 3 * b.layer;
+    float* g = a.sg ? a.sg + 3 * b.layer : nullptr;
+    if (b.uR > 0.0f) {
+        if (g) atomicAdd(g, w * X.kR * b.uR * pr);
+        a.gR = fmaf(w * __ldg(p), b.uR * pr, a.gR);
+    }
+    if (b.uM > 0.0f) {
+        if (g) atomicAdd(g + 1, w * X.omega * X.kM * b.uM * pm);
+        a.gW = fmaf(w * m.M, pm, a.gW);
+        a.gG = fmaf(w * m.Ms, slot.slope(), a.gG);
+        a.gM = fmaf(w * X.omega * __ldg(p + 1), b.uM * pm, a.gM);
+    }
 }
 // The coefficients at a vertex for its NEE terms and continuation.
 __device__ __forceinline__ AdjMed vertex_med(const AdjSet& X, const AdjBase& b) {
@@ -259,24 +287,19 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 acc.gR = acc.gM = acc.gO = acc_solar = 0.0f;
                 acc_band = band;
             }
-            // the segment integral of the ray that ended: an outgoing one's from its first
-            // random number, an unblocked shadow ray's from the position after its tracking
-            if (on && (meta & kFlagReplay)) {
-                const float4 H = P[kH], I = P[kI];
-                const AdjSet X = resolve(A.P, Lc, band);
-                const RayGeo g{RA.x, RA.y, RA.z};
-                float weight = 0.0f, t_end = RA.w;
-                Rng at = rng;
-                if (meta & kFlagShadow) {
-                    if (stage == kQContinue && state == kMiss) weight = H.w;
-                } else if (state == kHit || state == kMiss) {
-                    weight = I.x * X.kS * (H.z - P[kE].w);
-                    at.dim = as_u(I.z);
-                    if (state == kHit) t_end = B.x;
-                }
-                segment_terms(A, X, band, g, t_end, tau_bar, weight, at, acc);
-            }
         }
+        // the segment integral of the ray that ended: its weight, its end and its place in the random stream
+        float seg_weight = 0.0f, seg_end = RA.w;
+        uint32_t seg_dim = rng.dim;
+        if (kGrad && stage != kQTrack && on && (meta & kFlagReplay) && !(meta & kFlagShadow) &&
+            (state == kHit || state == kMiss)) {
+            // an outgoing ray's, from its first random number
+            const float4 I = P[kI];
+            seg_weight = I.x * resolve(A.P, Lc, band).kS * (P[kH].z - P[kE].w);
+            seg_dim = as_u(I.z);
+            if (state == kHit) seg_end = B.x;
+        }
+        const uint32_t seg_band = band;
 
         if (stage == kQTrack) {
             tracing = on;
@@ -289,14 +312,13 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 const V3 dir = mk(E.x, E.y, E.z);
                 float thr = D.w;
                 bool ground = (meta & kFlagGround) != 0u, alive = true;
-                AdjBase hb{0.0f, 0.0f, 0.0f, 0};
                 if (!(meta & kFlagShadow)) {  // a new vertex
                     ls = 0u;
                     ground = state != kHit;
                     if (!ground) {
                         const RayGeo g{RA.x, RA.y, RA.z};
                         org = madd(org, dir, B.x);
-                        hb = adj_base(S, band, altitude_at(g, B.x, S.ground_radius));
+                        const AdjBase hb = adj_base(S, band, altitude_at(g, B.x, S.ground_radius));
                         const AdjMed mq = adj_med(X, hb);
                         if (mq.t > 0.0f && mq.s > 0.0f) thr *= fminf(fmaxf(mq.s / mq.t, 0.0f), 1.0f);
                         alive = mq.t > 0.0f && mq.s > 0.0f && !(thr <= 0.0f);
@@ -306,9 +328,6 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                     }
                     P[kD] = make_float4(org.x, org.y, org.z, thr);
                     reinterpret_cast<float*>(&P[kF])[2] = 0.0f;  // the vertex's NEE sum
-                } else if (kGrad && !ground) {
-                    const float4 G = P[kG];
-                    hb = AdjBase{G.x, G.y, G.z, int(as_u(G.w))};
                 }
                 if (!alive) {
                     reinterpret_cast<float*>(&P[kE])[3] = fmaxf(E.w, 0.0f);
@@ -338,19 +357,6 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                     P[kB] = B;
                     reinterpret_cast<float*>(&P[kC])[2] = as_f(meta);
                     reinterpret_cast<float*>(&P[kC])[3] = as_f(job | (ls << 16));
-                    if (kGrad && set_up) {
-                        // the term ahead of its ray: it weighs the ray's segment integral
-                        const float mu = P[kF].w, l_sun = __ldg(&S.bands[band].solar_radiance);
-                        float term;
-                        if (ground) {
-                            term = S.ground_albedo * kInvPi * l_sun * mu / S.light_pdf;
-                        } else {
-                            term = l_sun * nee_phase(X, bins, vertex_med(X, hb), mu) / S.light_pdf;
-                        }
-                        const float w = P[kI].x * X.kS;
-                        reinterpret_cast<float*>(&P[kH])[3] = w * thr * term * (1.0f / float(lights));
-                        reinterpret_cast<float*>(&P[kI])[1] = term;
-                    }
                 }
             }
         } else if (stage == kQContinue) {
@@ -368,55 +374,73 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 }
                 const AdjMed mq = vertex_med(X, hb);
                 const uint32_t lights = L.direct_light_samples;
-                if (state == kMiss) {  // the sample's term, transmittance 1 (sky_trace.wgsl:566-608)
-                    if (kGrad) {
-                        nee += P[kI].y;
-                        if (replay && !ground) vertex_terms(acc, X, bins, hb, mq, F.w, P[kH].w);
-                    } else {
-                        const float mu = F.w, l_sun = __ldg(&S.bands[band].solar_radiance);
-                        float term;
-                        if (ground) {
-                            term = S.ground_albedo * kInvPi * l_sun * mu / S.light_pdf;
-                        } else {
-                            term = l_sun * nee_phase(X, bins, mq, mu) / S.light_pdf;
-                        }
-                        nee = __fadd_rn(nee, term);  // not contracted into the term's division
-                    }
+                const bool lit = state == kMiss, more_lights = ls < lights;
+                const float w = kGrad ? P[kI].x * X.kS : 0.0f;
+                float thr = D.w, rad = E.w;
+                V3 nd = mk(0.0f, 1.0f, 0.0f), axis = dir;
+                float cos_t = 1.0f, sin_t = 0.0f, xi_phi = 0.0f;
+                bool framed = true;
+                if (lit && ground) {
+                    const float term =
+                        S.ground_albedo * kInvPi * __ldg(&S.bands[band].solar_radiance) * F.w / S.light_pdf;
+                    nee = __fadd_rn(nee, term);
+                    if (kGrad) seg_weight = w * thr * term * (1.0f / float(lights));
                 }
-                if (ls < lights) {
-                    reinterpret_cast<float*>(&P[kF])[2] = nee;
-                    next = kQVertex;
-                } else {
-                    float thr = D.w, rad = E.w;
-                    uint32_t depth = as_u(F.x);
-                    rad += thr * (nee * (1.0f / float(lights)));
-                    // each branch draws its angles; one shared frame step turns them into
-                    // the direction (as direction_from_axis_mu / sample_cosine_hemisphere)
-                    V3 nd = mk(0.0f, 1.0f, 0.0f), axis = dir;
-                    float cos_t = 1.0f, sin_t = 0.0f, xi_phi = 0.0f;
-                    bool framed = true;
-                    if (!ground) {
-                        float mu_c, fq;
+                // the phase function at a medium vertex, once for the lit sun sample's term (its
+                // transmittance is 1, sky_trace.wgsl:566-608) and once for the continuation,
+                // by the same code (one copy of it in the gradient, whose code is large: 3.44 ->
+                // 3.09 ms; two in the primal, where one is 5 % slower)
+                constexpr int kCopies = kGrad ? 1 : 2;
+#pragma unroll kCopies
+                for (uint32_t k = 0u; k < 2u; ++k) {
+                    float mu = F.w, pdf = 1.0f;
+                    if (k == 0u) {
+                        if (ground || !lit) continue;
+                    } else {
+                        if (more_lights) break;
+                        rad += thr * (nee * (1.0f / float(lights)));
+                        if (ground) break;
                         if (kPhase == SKY_PHASE_TABULATED) {
                             const float target = rng.next() * mq.s;
                             const bool rayleigh = target < mq.R || !(mq.Ms > 0.0f);
                             const float xi_mu = rng.next();
-                            mu_c = rayleigh ? invert_rayleigh_cdf(xi_mu) : hg_sample_mu(X, bins, xi_mu);
+                            mu = rayleigh ? invert_rayleigh_cdf(xi_mu) : hg_sample_mu(X, bins, xi_mu);
                             xi_phi = rng.next();
-                            cos_t = fminf(fmaxf(mu_c, -1.0f), 1.0f);
+                            cos_t = fminf(fmaxf(mu, -1.0f), 1.0f);
                             sin_t = sqrtf(fmaxf(1.0f - cos_t * cos_t, 0.0f));
-                            const float pdf = mixed(mq, rayleigh_phase(mu_c),
-                                                    mq.Ms > 0.0f ? hg_sampling_pdf(X, bins, mu_c) : 0.0f);
-                            fq = mixed_phase_value(X, bins, mq, mu_c) / pdf;
+                            pdf = mixed(mq, rayleigh_phase(mu), mq.Ms > 0.0f ? hg_sampling_pdf(X, bins, mu) : 0.0f);
                         } else {
                             nd = sample_isotropic(rng);
                             framed = false;
-                            mu_c = dot3(dir, nd);
-                            fq = mixed_phase_value(X, bins, mq, mu_c) / mq.s / kIsotropicPdf;
+                            mu = dot3(dir, nd);
                         }
-                        thr *= fq;
-                        if (replay) vertex_terms(acc, X, bins, hb, mq, mu_c, P[kI].x * X.kS * (P[kH].z - rad));
+                    }
+                    const HgSlot slot(X, bins, mu);
+                    const float pr = rayleigh_phase(mu), pm = mq.Ms > 0.0f ? slot.value() : 0.0f;
+                    float weight;
+                    if (k == 0u) {
+                        const float sum = __fadd_rn(__fmul_rn(mq.R, pr), mq.Ms > 0.0f ? __fmul_rn(mq.Ms, pm) : 0.0f);
+                        const float ph = mq.s > 0.0f ? sum / mq.s : 0.0f;
+                        const float term = __ldg(&S.bands[band].solar_radiance) * ph / S.light_pdf;
+                        nee = __fadd_rn(nee, term);  // not contracted into the term's division
+                        weight = kGrad ? w * thr * term * (1.0f / float(lights)) : 0.0f;
+                        if (kGrad) seg_weight = weight;
                     } else {
+                        const float value = mixed(mq, pr, pm);
+                        thr *= kPhase == SKY_PHASE_TABULATED ? value / pdf : value / mq.s / kIsotropicPdf;
+                        weight = kGrad ? w * (P[kH].z - rad) : 0.0f;
+                    }
+                    if (replay) vertex_terms_at(acc, X, slot, hb, mq, pr, weight);
+                }
+                if (kGrad && !replay) seg_weight = 0.0f;
+                if (more_lights) {
+                    reinterpret_cast<float*>(&P[kF])[2] = nee;
+                    next = kQVertex;
+                } else {
+                    uint32_t depth = as_u(F.x);
+                    // each branch has drawn its angles; one shared frame step turns them into
+                    // the direction (as direction_from_axis_mu / sample_cosine_hemisphere)
+                    if (ground) {
                         // the Lambert bounce (sky_trace.wgsl:750-766)
                         axis = normalize_or_y(org);
                         const float u = rng.next();
@@ -582,6 +606,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
             }
         }
 
+        if (kGrad && seg_weight != 0.0f) {
+            Rng at = rng;
+            at.dim = seg_dim;
+            at.k0 = as_u(C.x);
+            at.k1 = as_u(C.y);
+            at.k2 = seg_band * 1664525u + 1013904223u;
+            const RayGeo g{RA.x, RA.y, RA.z};
+            segment_terms(A, resolve(A.P, Lc, seg_band), seg_band, g, seg_end, tau_bar, seg_weight, at, acc);
+        }
         // the stages' rays, as the tracer sets them up
         if (set_up) {
             const RayGeo g = ray_geo(ray_org, ray_dir);
@@ -675,7 +708,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 template <int kPhase, bool kGrad, bool kBatchOfRenders>
 cudaError_t launch_shape(const AdjCtx& A, const AdjJobs& J, double* layer_grad, double* band_grad, uint32_t* status,
                          unsigned long long* work_counter, cudaStream_t stream) {
-    constexpr int kWarps = kGrad ? 12 : 16;  // 80 and 64 registers per lane
+        constexpr int kWarps = kGrad ? 12 : 16;  // 80 and 64 registers per lane
     constexpr uint32_t kThreads = kWarps * 32u;
     const void* k = reinterpret_cast<const void*>(adjoint_wave_kernel<kPhase, kGrad, kBatchOfRenders, kWarps>);
     int dev = 0, sms = 0, per_sm = 0, smem_sm = 0, smem_block = 0, reserved = 0;
