@@ -143,17 +143,27 @@ void build_phase_sampling_tables(const float* values, uint32_t band_count, uint3
         float u = float(e) / float(bins);
         return 1.0f - 2.0f * u * u * u;
     };
+    std::vector<float> width(bins);  // of the cube-root mu bins
+    for (uint32_t bin = 0; bin < bins; ++bin) width[bin] = std::fabs(edge(bin) - edge(bin + 1));
     for (uint32_t species = 0; species < kSpecies; ++species) {
         for (uint32_t band = 0; band < band_count; ++band) {
             size_t base = (size_t(species) * band_count + band) * bins;
+            // a row equal to the one before it (a species without aerosol, a table that does
+            // not vary with the wavelength) has that row's tables
+            if (base && std::memcmp(values + base, values + base - bins, bins * sizeof(float)) == 0) {
+                std::copy_n(cdf.begin() + (base - bins), bins, cdf.begin() + base);
+                std::copy_n(bin_pdf.begin() + (base - bins), bins, bin_pdf.begin() + base);
+                if (guide) std::copy_n(guide->begin() + (base - bins), bins, guide->begin() + base);
+                continue;
+            }
             float norm = 0.0f;
             for (uint32_t bin = 0; bin < bins; ++bin)
-                norm += 2.0f * kPiF * std::max(values[base + bin], 0.0f) * std::fabs(edge(bin) - edge(bin + 1));
+                norm += 2.0f * kPiF * std::max(values[base + bin], 0.0f) * width[bin];
             norm = std::max(norm, 1.0e-20f);
             float cumulative = 0.0f;
             for (uint32_t bin = 0; bin < bins; ++bin) {
                 float value = std::max(values[base + bin], 0.0f);
-                cumulative += 2.0f * kPiF * value * std::fabs(edge(bin) - edge(bin + 1)) / norm;
+                cumulative += 2.0f * kPiF * value * width[bin] / norm;
                 cdf[base + bin] = std::min(cumulative, 1.0f);
                 bin_pdf[base + bin] = value / norm;
             }
@@ -176,20 +186,28 @@ void build_phase_sampling_tables(const float* values, uint32_t band_count, uint3
 std::vector<uint32_t> merge_majorant_layers(const float* maj, uint32_t L, float dz, double crossing_cost) {
     std::vector<double> best(L + 1, 0.0);
     std::vector<uint32_t> from(L + 1, 0);
+    std::vector<double> floor_maj(L);
+    for (uint32_t i = 0; i < L; ++i) floor_maj[i] = std::max(double(maj[i]), 1e-8);
+    const double ddz = double(dz);
     for (uint32_t j = 1; j <= L; ++j) {
-        best[j] = 1e300;
-        double mx = 0.0, sum = 0.0;
+        double least = 1e300, mx = 0.0, sum = 0.0, n = 0.0;
+        uint32_t at = 0;
         for (uint32_t i = j; i-- > 0;) {  // group [i, j)
-            double m = std::max(double(maj[i]), 1e-8);
+            const double m = floor_maj[i];
+            n += 1.0;
             mx = std::max(mx, m);
             sum += m;
-            double excess = (mx * double(j - i) - sum) * double(dz);
-            double c = best[i] + crossing_cost + excess;
-            if (c < best[j]) {
-                best[j] = c;
-                from[j] = i;
+            const double excess = (mx * n - sum) * ddz;
+            // a larger group has at least this excess (up to rounding, far below the margin)
+            if (crossing_cost + excess > least * (1.0 + 1e-6) + 1e-6 * mx * double(L) * ddz) break;
+            const double c = best[i] + crossing_cost + excess;
+            if (c < least) {
+                least = c;
+                at = i;
             }
         }
+        best[j] = least;
+        from[j] = at;
     }
     std::vector<uint32_t> starts;
     for (uint32_t j = L; j > 0; j = from[j]) starts.push_back(from[j]);

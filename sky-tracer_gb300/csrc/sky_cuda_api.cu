@@ -35,7 +35,8 @@ struct SkyScene {
     bool has_xyz = false;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
-    // workspace
+    // workspace: one allocation, and its parts
+    unsigned char* ws = nullptr;
     double* ws_sum = nullptr;
     double* ws_sumsq = nullptr;
     float* ws_film = nullptr;
@@ -111,54 +112,54 @@ uint32_t slab_rows(const SkyRenderConfig* c) { return c->row_count ? c->row_coun
 uint64_t slab_pixels(const SkyRenderConfig* c) { return uint64_t(c->width) * slab_rows(c); }
 
 void free_workspace(SkyScene* s) {
-    cudaFree(s->ws_sum);
-    cudaFree(s->ws_sumsq);
-    cudaFree(s->ws_film);
-    cudaFree(s->ws_xyz);
-    cudaFree(s->ws_xyz_var);
-    cudaFree(s->ws_rgb);
-    s->ws_rgb = nullptr;
-    cudaFree(s->ws_counters);
-    cudaFree(s->ws_status);
+    cudaFree(s->ws);
+    s->ws = nullptr;
     s->ws_sum = s->ws_sumsq = nullptr;
-    s->ws_film = nullptr;
+    s->ws_film = s->ws_rgb = nullptr;
     s->ws_xyz = s->ws_xyz_var = nullptr;
     s->ws_counters = nullptr;
     s->ws_status = nullptr;
     s->ws_cells = s->ws_pixels = 0;
 }
 
-// Grow the render workspace to `pixels`.  The new buffers are allocated
-// before the old ones are freed, so a failed allocation leaves the scene with
+// A render's event counts and status word: cleared by one memset, read by one copy.
+struct Diagnostics {
+    unsigned long long counters[SKY_EVENT_COUNT];
+    uint32_t status;
+};
+
+// Grow the render workspace to `pixels`, in one allocation.  The new one is
+// made before the old one is freed, so a failed allocation leaves the scene with
 // its old workspace: renders that fit it still run without allocating.
 int ensure_workspace(SkyScene* s, uint64_t pixels) {
-    uint64_t cells = pixels * s->dev.band_count;
+    const uint64_t cells = pixels * s->dev.band_count;
     if (cells <= s->ws_cells && pixels <= s->ws_pixels && s->ws_sum) return SKY_OK;
-    SkyScene grown;
-    grown.dev = s->dev;
-    cudaError_t e = cudaSuccess;
-    if ((e = dev_malloc(&grown.ws_sum, cells * sizeof(double))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_sumsq, cells * sizeof(double))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_film, cells * sizeof(float))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_xyz, pixels * 3 * sizeof(double))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_xyz_var, pixels * 3 * sizeof(double))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_rgb, pixels * 3 * sizeof(float))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_counters, SKY_EVENT_COUNT * sizeof(unsigned long long))) != cudaSuccess ||
-        (e = dev_malloc(&grown.ws_status, sizeof(uint32_t))) != cudaSuccess) {
-        free_workspace(&grown);
-        return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "workspace allocation", e);
-    }
+    size_t off = 0;
+    auto reserve = [&off](size_t bytes) {
+        const size_t at = off;
+        off = align_up(off + bytes, 256);
+        return at;
+    };
+    const size_t o_sum = reserve(cells * sizeof(double)), o_sumsq = reserve(cells * sizeof(double)),
+                 o_film = reserve(cells * sizeof(float)), o_xyz = reserve(pixels * 3 * sizeof(double)),
+                 o_var = reserve(pixels * 3 * sizeof(double)), o_rgb = reserve(pixels * 3 * sizeof(float)),
+                 o_counters = reserve(sizeof(Diagnostics));
+    unsigned char* base = nullptr;
+    const cudaError_t e = dev_malloc(&base, off);
+    if (e != cudaSuccess) return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "workspace allocation", e);
     // the old buffers may still be read by work queued on the scene's stream
-    if (s->stream) cudaStreamSynchronize(s->stream);
+    if (s->ws && s->stream) cudaStreamSynchronize(s->stream);
     free_workspace(s);
-    s->ws_sum = grown.ws_sum;
-    s->ws_sumsq = grown.ws_sumsq;
-    s->ws_film = grown.ws_film;
-    s->ws_xyz = grown.ws_xyz;
-    s->ws_xyz_var = grown.ws_xyz_var;
-    s->ws_rgb = grown.ws_rgb;
-    s->ws_counters = grown.ws_counters;
-    s->ws_status = grown.ws_status;
+    s->ws = base;
+    s->ws_sum = reinterpret_cast<double*>(base + o_sum);
+    s->ws_sumsq = reinterpret_cast<double*>(base + o_sumsq);
+    s->ws_film = reinterpret_cast<float*>(base + o_film);
+    s->ws_xyz = reinterpret_cast<double*>(base + o_xyz);
+    s->ws_xyz_var = reinterpret_cast<double*>(base + o_var);
+    s->ws_rgb = reinterpret_cast<float*>(base + o_rgb);
+    Diagnostics* diagnostics = reinterpret_cast<Diagnostics*>(base + o_counters);
+    s->ws_counters = diagnostics->counters;
+    s->ws_status = &diagnostics->status;
     s->ws_cells = cells;
     s->ws_pixels = pixels;
     return SKY_OK;
@@ -363,8 +364,7 @@ int render_host(SkyScene* s, const SkyRenderConfig* c, float* film_out, size_t f
     if (cudaSetDevice(s->device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "cannot select the device");
     if ((st = ensure_workspace(s, pixels))) return st;
     cudaError_t e;
-    e = cudaMemsetAsync(s->ws_counters, 0, SKY_EVENT_COUNT * sizeof(unsigned long long), s->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->ws_status, 0, sizeof(uint32_t), s->stream);
+    e = cudaMemsetAsync(s->ws_counters, 0, sizeof(Diagnostics), s->stream);
     if (e != cudaSuccess) return cuda_fail(SKY_ERR_LAUNCH, "clearing counters", e);
     // events are counted only when the caller asks for them (counting costs the wavefront kernel ~3 %)
     const bool count = stats && (c->flags & SKY_FLAG_COUNT_EVENTS) != 0;
@@ -372,8 +372,7 @@ int render_host(SkyScene* s, const SkyRenderConfig* c, float* film_out, size_t f
                        xyz_var_out ? s->ws_xyz_var : nullptr, count ? s->ws_counters : nullptr, s->ws_status,
                        rgb_out ? s->ws_rgb : nullptr};
     if ((st = launch_render(s, c, &o, s->stream, true))) return st;
-    uint32_t status = 0;
-    unsigned long long counters[SKY_EVENT_COUNT] = {};
+    Diagnostics found{};
     if (film_out &&
         (e = cudaMemcpyAsync(film_out, s->ws_film, cells * sizeof(float), cudaMemcpyDeviceToHost, s->stream)))
         return cuda_fail(SKY_ERR_COPY, "film readback", e);
@@ -386,16 +385,16 @@ int render_host(SkyScene* s, const SkyRenderConfig* c, float* film_out, size_t f
     if (rgb_out &&
         (e = cudaMemcpyAsync(rgb_out, s->ws_rgb, pixels * 3 * sizeof(float), cudaMemcpyDeviceToHost, s->stream)))
         return cuda_fail(SKY_ERR_COPY, "rgb readback", e);
-    if ((e = cudaMemcpyAsync(counters, s->ws_counters, sizeof(counters), cudaMemcpyDeviceToHost, s->stream)) ||
-        (e = cudaMemcpyAsync(&status, s->ws_status, sizeof(status), cudaMemcpyDeviceToHost, s->stream)))
+    if ((e = cudaMemcpyAsync(&found, s->ws_counters, sizeof(found), cudaMemcpyDeviceToHost, s->stream)))
         return cuda_fail(SKY_ERR_COPY, "diagnostics readback", e);
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return cuda_fail(SKY_ERR_SYNC, "waiting for the GPU", e);
+    const uint32_t status = found.status;
     if (stats) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, s->ev_start, s->ev_stop);
         stats->kernel_ms = ms;
         stats->chains = uint64_t(cells) * c->spp;
-        for (int i = 0; i < SKY_EVENT_COUNT; ++i) stats->events[i] = counters[i];
+        for (int i = 0; i < SKY_EVENT_COUNT; ++i) stats->events[i] = found.counters[i];
         stats->watchdog = status;
         stats->kernel_used = c->kernel == SKY_KERNEL_PLAIN ? SKY_KERNEL_PLAIN : SKY_KERNEL_WAVEFRONT;
         stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -626,11 +625,14 @@ int sky_cuda_scene_create(const SkySceneDesc* desc, SkyScene** out_scene) {
             s->adjoint_unsupported = "differentiable renders need a scene whose only aerosol is species 0; species " +
                                      std::to_string(sp) + " has mass and optics";
     }
-    if ((e = dev_malloc(&s->jobs, sizeof(DevJob))) != cudaSuccess ||
-        (e = dev_malloc(&s->work_counter, sizeof(*s->work_counter))) != cudaSuccess) {
+    // one job row, with the work counter behind it
+    const size_t job_bytes = align_up(sizeof(DevJob), sizeof(*s->work_counter));
+    if ((e = dev_malloc(&s->jobs, job_bytes + sizeof(*s->work_counter))) != cudaSuccess) {
         sky_cuda_scene_destroy(s);
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "job table allocation", e);
     }
+    s->work_counter =
+        reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(s->jobs) + job_bytes);
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreate(&s->ev_start)) != cudaSuccess || (e = cudaEventCreate(&s->ev_stop)) != cudaSuccess) {
         sky_cuda_scene_destroy(s);
@@ -651,7 +653,6 @@ void sky_cuda_scene_destroy(SkyScene* s) {
     cudaFree(s->trk_blob);
     cudaFree(s->adj_ws);
     cudaFree(s->jobs);
-    cudaFree(s->work_counter);
     cudaFree(s->blob);
     if (s->ev_start) cudaEventDestroy(s->ev_start);
     if (s->ev_stop) cudaEventDestroy(s->ev_stop);

@@ -43,6 +43,7 @@ struct WaveLaunch {
     unsigned long long* counters;  // may be null
     uint32_t* status;
     uint32_t iteration_limit;      // loop iterations per warp before status bit 2 (SkyTuning.iteration_limit)
+    int sms;                       // SMs of the current device (filled in by launch_trace_wave)
 };
 
 // Prepare, trace and finalize every job of `w` (three kernels on `stream`):

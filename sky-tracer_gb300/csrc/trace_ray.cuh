@@ -416,10 +416,9 @@ template <int kTracking, int kPhase, bool kSingle, bool kCount, int kAer>
 cudaError_t launch_ray_shape(const WaveLaunch& w, cudaStream_t stream) {
     const void* k =
         reinterpret_cast<const void*>(ray_kernel<kTracking, kPhase, kSingle, kCount, kAer>);
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, per_sm = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     // the staged medium tables and the vertex cache: 12.7 KB for 81 bands over 68 knots and one
     // aerosol species; the largest scenes the library accepts (1024 knots, 256 bands) need 77 KB,
     // beyond the 48 KB a launch gets without opting in
@@ -447,7 +446,7 @@ cudaError_t launch_ray_shape(const WaveLaunch& w, cudaStream_t stream) {
     if (w.max_blocks_per_sm) per_sm = std::min(per_sm, int(w.max_blocks_per_sm));
     // a warp per cell at most
     const uint64_t want = (uint64_t(w.total_cells) * 32u + kWaveThreads - 1u) / kWaveThreads;
-    const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * sms, want)));
+    const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * uint64_t(w.sms), want)));
     ray_kernel<kTracking, kPhase, kSingle, kCount, kAer><<<blocks, kWaveThreads, smem, stream>>>(
         w.scene, w.launch0, w.jobs, w.num_jobs, w.total_cells, reinterpret_cast<uint32_t*>(w.work_counter), w.counters, w.status,
         w.iteration_limit ? w.iteration_limit : kMaxIterations);

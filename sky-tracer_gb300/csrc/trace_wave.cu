@@ -35,29 +35,29 @@ __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restr
 //                      four: 4.0 M 1.47 / 1.60, 5.4 M 1.86 / 1.81: 34 per lane
 //   residual carry     131 k 0.52 / 0.68, 262 k 0.63 / 0.62, 524 k 0.82 / 0.70: 2 per lane
 //   segment restart    0.67 M 1.25 / 1.34, 1.0 M 1.63 / 1.12: 5 per lane
-cudaError_t small_render(const WaveLaunch& w, bool& small) {
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+bool small_render(const WaveLaunch& w) {
     const uint64_t per_lane = w.tracking == SKY_TRACKING_SEGMENT_RESTART  ? 5u
                               : w.tracking == SKY_TRACKING_RESIDUAL_CARRY ? 2u
                               : w.aerosol_species == 1u                   ? 24u
                                                                           : 34u;
-    small = w.total_chains < per_lane * 1024u * uint64_t(sms);
-    return e;
+    return w.total_chains < per_lane * 1024u * uint64_t(w.sms);
 }
 
 }  // namespace
 
-cudaError_t launch_trace_wave(const WaveLaunch& w, cudaStream_t stream) {
+cudaError_t launch_trace_wave(const WaveLaunch& asked, cudaStream_t stream) {
+    WaveLaunch w = asked;
     if (w.num_jobs == 0u || w.num_jobs > 65535u || w.total_cells == 0u) return cudaErrorInvalidValue;
     const uint32_t xblocks =
         uint32_t(std::min<uint64_t>((uint64_t(w.max_job_cells) + 255u) / 256u, 1024u));
     wave_prepare_kernel<<<dim3(std::max(xblocks, 1u), w.num_jobs), 256, 0, stream>>>(w.jobs, w.work_counter);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    bool small = false;
-    if ((e = small_render(w, small)) != cudaSuccess) return e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&w.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    const bool small = small_render(w);
     switch (w.tracking) {
         case SKY_TRACKING_SEGMENT_RESTART:
             e = small ? launch_ray_segment_restart(w, stream) : launch_wave_segment_restart(w, stream);

@@ -663,10 +663,9 @@ cudaError_t launch_wave_shape(const WaveLaunch& w, cudaStream_t stream) {
     const void* k =
         reinterpret_cast<const void*>(wave_kernel<kTracking, kPhase, kWarps, kSingle, kCount, kAer>);
     constexpr uint32_t kThreads = kWarps * 32u;
-    int dev = 0, sms = 0, per_sm = 0, smem_sm = 0, smem_block = 0, reserved = 0;
+    int dev = 0, per_sm = 0, smem_sm = 0, smem_block = 0, reserved = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess)
         return e;
     if ((e = cudaDeviceGetAttribute(&smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
@@ -701,7 +700,7 @@ cudaError_t launch_wave_shape(const WaveLaunch& w, cudaStream_t stream) {
     if (w.max_blocks_per_sm) per_sm = std::min(per_sm, int(w.max_blocks_per_sm));
     // a warp of chains per block at least; a small render spreads its chains over the blocks
     const uint64_t want = (w.total_chains + 31u) / 32u;
-    const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * sms, want)));
+    const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * uint64_t(w.sms), want)));
     const uint64_t share = ((w.total_chains + blocks - 1u) / blocks + 31u) / 32u * 32u;
     const uint32_t used = uint32_t(std::min<uint64_t>(paths, share));
     const uint32_t limit = uint32_t(std::min<uint64_t>(
