@@ -625,8 +625,10 @@ int sky_cuda_scene_create(const SkySceneDesc* desc, SkyScene** out_scene) {
             s->adjoint_unsupported = "differentiable renders need a scene whose only aerosol is species 0; species " +
                                      std::to_string(sp) + " has mass and optics";
     }
-    // one job row, with the work counter behind it
-    const size_t job_bytes = align_up(sizeof(DevJob), sizeof(*s->work_counter));
+    // one job row, and behind it the work counter in a cache line of its own: sharing the row's, its
+    // atomics slow the row's readers (509x251, 79 bands, 3 spp: 4.07 against 3.69 ms; production 295.5
+    // against 289.6 ms)
+    const size_t job_bytes = align_up(sizeof(DevJob), 256);
     if ((e = dev_malloc(&s->jobs, job_bytes + sizeof(*s->work_counter))) != cudaSuccess) {
         sky_cuda_scene_destroy(s);
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "job table allocation", e);
@@ -1470,7 +1472,7 @@ namespace {
 
 struct NoAllocScratch {
     DevJob jobs[SKY_NOALLOC_MAX_JOBS];
-    unsigned long long work_counter;
+    alignas(256) unsigned long long work_counter;  // a cache line of its own, apart from the rows that are read
 };
 static_assert(sizeof(NoAllocScratch) <= SKY_NOALLOC_SCRATCH_BYTES, "scratch area too small");
 
