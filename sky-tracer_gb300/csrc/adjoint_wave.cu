@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float* const grads = reinterpret_cast<float*>(
         smem + align16(size_t(paths) * kRows * 16u + sizeof(Queues) + size_t(kQueues) * queue_slots(paths) * 2u));
-    float* const sg = kGrad && layer_grad ? grads + (warp % copies) * nlayer : nullptr;
+    float* const sg = kGrad && copies ? grads + (warp * 2u + (lane & 1u)) % copies * nlayer : nullptr;
     float* const sb = grads + copies * nlayer;
     for (uint32_t i = threadIdx.x; i < used_paths; i += blockDim.x)
         pool[i * kRows + kB] = make_float4(0.0f, as_f(kFresh), 0.0f, 0.0f);
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 template <int kPhase, bool kGrad, bool kBatchOfRenders>
 cudaError_t launch_shape(const AdjCtx& A, const AdjJobs& J, double* layer_grad, double* band_grad, uint32_t* status,
                          unsigned long long* work_counter, cudaStream_t stream) {
-        constexpr int kWarps = kGrad ? 12 : 16;  // 80 and 64 registers per lane
+    constexpr int kWarps = kGrad ? 12 : 16;  // 80 and 64 registers per lane
     constexpr uint32_t kThreads = kWarps * 32u;
     const void* k = reinterpret_cast<const void*>(adjoint_wave_kernel<kPhase, kGrad, kBatchOfRenders, kWarps>);
     int dev = 0, sms = 0, per_sm = 0, smem_sm = 0, smem_block = 0, reserved = 0;
@@ -719,9 +719,16 @@ cudaError_t launch_shape(const AdjCtx& A, const AdjJobs& J, double* layer_grad, 
         (e = cudaDeviceGetAttribute(&smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess)
         return e;
-    // one layer-gradient copy per warp while two blocks of them leave the paths room, else one
+    // two layer-gradient copies per warp, of its even and its odd lanes (an FP32 addition in shared
+    // memory is repeated for each lane that meets another at its address; 16.8 M chains, 64 layers: one
+    // 3.09, two 3.00, four 2.98 ms), while two blocks of them leave the paths room; else one per
+    // warp, or one
     const size_t nlayer = 3u * A.S.layer_count + 2u, nband = kGrad ? size_t(kAdjBandParams) * A.S.band_count : 0u;
-    const uint32_t copies = kGrad ? (kWarps * nlayer * sizeof(float) <= 16u * 1024u ? uint32_t(kWarps) : 1u) : 0u;
+    const size_t warp_copy = kWarps * nlayer * sizeof(float);
+    const uint32_t copies = !kGrad || !layer_grad         ? 0u
+                            : warp_copy <= 12u * 1024u ? 2u * uint32_t(kWarps)
+                            : warp_copy <= 16u * 1024u ? uint32_t(kWarps)
+                                                       : 1u;
     const size_t extra = (copies * nlayer + nband) * sizeof(float);
     auto bytes = [&](uint32_t p) {
         return align16(size_t(p) * path_rows<kGrad>() * 16u + sizeof(Queues) +
@@ -749,7 +756,7 @@ cudaError_t launch_shape(const AdjCtx& A, const AdjJobs& J, double* layer_grad, 
     const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(std::max(per_sm, 1)) * sms, want)));
     const uint32_t used = uint32_t(std::min<uint64_t>(paths, ((J.chains + blocks - 1u) / blocks + 31u) / 32u * 32u));
     adjoint_wave_kernel<kPhase, kGrad, kBatchOfRenders, kWarps><<<blocks, kThreads, smem, stream>>>(
-        A, J, layer_grad, band_grad, paths, used, std::max(copies, 1u), work_counter, status);
+        A, J, layer_grad, band_grad, paths, used, copies, work_counter, status);
     return cudaGetLastError();
 }
 

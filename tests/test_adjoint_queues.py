@@ -118,3 +118,26 @@ def test_a_batch_takes_the_queues(gpu, data_dir):
         one = [r.backward(layer, band, dloss, sun=s) for s in suns]
         for x, y in ((lg, one[0][0] + one[1][0]), (bg, one[0][1] + one[1][1])):
             assert float((x - y).abs().max()) <= 2e-4 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("layers", [84, 85, 113, 114])
+def test_layer_gradient_copies(gpu, data_dir, layers):
+    """Two copies of the layer gradient per warp up to 84 layers, one up to 113, one per block above."""
+    import torch
+    scene = synthetic_scene(wavelengths(420.0, 680.0, 6), data_dir, sun_elevation_deg=25.0).bake_majorants(layers)
+    spp = -(-_chains(True) // (32 * 16 * 6)) + 1
+    cfg = RenderConfig(width=32, height=16, spp=spp, phase_sampling=_abi.PHASE_TABULATED,
+                       tracking=_abi.TRACKING_MERGED_LAYERS, seed=8)
+    with GpuScene(scene) as gs:
+        r = AdjointRenderer(gs, cfg)
+        assert r.param_count == 3 * layers + 2
+        layer = torch.ones(r.param_count, device="cuda")
+        layer[-2], layer[-1] = 0.9, 0.76
+        band = torch.ones((6, 4), device="cuda")
+        dloss = torch.ones((16, 32, 6), device="cuda")
+        chains = r.new_chain_buffer()
+        _forward(r, layer, band, chains, None)
+        count = torch.zeros(8, dtype=torch.int64, device="cuda")
+        for x, y in zip(_backward(r, layer, band, dloss, chains, None),
+                        _backward(r, layer, band, dloss, chains, count)):
+            assert np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
