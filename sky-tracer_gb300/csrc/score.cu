@@ -23,10 +23,13 @@
 // three times: the first histogram is now taken while the distances are made,
 // the others from one reading for all five, of a buffer that stays in L2.
 // 655 360 samples x 128 combinations of 4 bands: 5.9 ms of kernels and four
-// round trips to the host -> 1.8 ms (distances 0.85, histograms 0.74, picks 0.18)
-// and one.  The reference's scale and Oklab (0.34 ms here) took 33 ms on the host.
+// round trips to the host -> 1.3 ms (distances 0.80, histograms 0.36, picks 0.13)
+// and one.  The reference's scale and Oklab (0.18 ms here) took 33 ms on the host.
+// One distance at a time per thread, one target's scan after the other in the
+// picks, and one warp for the scale's: 1.8 and 0.34 ms.
 
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -53,7 +56,7 @@ __device__ __forceinline__ void xyz_to_oklab(float x, float y, float z, float la
 }
 
 // Combinations of a block, and samples of a thread in a tile.
-constexpr uint32_t kCombos = 4, kSamples = 4;
+constexpr uint32_t kCombos = kScoreGroup, kSamples = 4;
 constexpr uint32_t kTile = 256u * kSamples;
 
 // A sum kept as an unevaluated pair of floats.  Each addition's rounding error
@@ -178,7 +181,9 @@ __global__ void __launch_bounds__(256) distance_kernel(const float* __restrict__
 
 // Histograms of the next `width` bits of combination blockIdx.y's distances,
 // one for each of its targets' prefixes (the bits above `shift + width`).
-// Targets with the same prefix share the first one's.
+// Targets with the same prefix share the first one's.  A thread reads four
+// distances at a time (one at a time, the last digit's reading, which finds almost
+// none of its prefixes, took 67 us for 65 MB of L2).
 __global__ void __launch_bounds__(256) select_hist_kernel(const float* __restrict__ dist, uint64_t samples,
                                                           const ScoreState* __restrict__ state, uint32_t shift,
                                                           uint32_t width, uint32_t* __restrict__ hist) {
@@ -188,22 +193,29 @@ __global__ void __launch_bounds__(256) select_hist_kernel(const float* __restric
     if (S.count == 0u) return;
     uint32_t prefix[kScoreTargets];
 #pragma unroll
-    for (uint32_t t = 0; t < kScoreTargets; ++t) prefix[t] = S.prefix[t];
+    for (uint32_t t = kScoreTargets; t-- > 0u;)  // 0xffffffff: no distance has it
+        prefix[t] = t && S.prefix[t] == S.prefix[t - 1u] ? 0xffffffffu : S.prefix[t];
     for (uint32_t i = threadIdx.x; i < kScoreTargets * kScoreHistBins; i += blockDim.x) (&h[0][0])[i] = 0u;
     __syncthreads();
     const float* row = dist + size_t(c) * samples;
-    for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < samples;
-         s += uint64_t(gridDim.x) * blockDim.x) {
-        const float e = __ldg(row + s);
-        if (!(e == e)) continue;  // NaN
-        const uint32_t bits = __float_as_uint(e), above = bits >> top, digit = (bits >> shift) & (bins - 1u);
+    for (uint64_t tile = uint64_t(blockIdx.x) * kTile; tile < samples; tile += uint64_t(gridDim.x) * kTile) {
+        uint32_t bits[kSamples];
 #pragma unroll
-        for (uint32_t t = 0; t < kScoreTargets; ++t)
-            if (above == prefix[t] && (t == 0u || prefix[t] != prefix[t - 1u])) atomicAdd(&h[t][digit], 1u);
+        for (uint32_t j = 0; j < kSamples; ++j) {
+            const uint64_t s = tile + j * 256u + threadIdx.x;
+            bits[j] = s < samples ? __float_as_uint(__ldg(row + s)) : 0x7fffffffu;  // NaN: above every prefix
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kSamples; ++j) {
+            const uint32_t above = bits[j] >> top, digit = (bits[j] >> shift) & (bins - 1u);
+#pragma unroll
+            for (uint32_t t = 0; t < kScoreTargets; ++t)
+                if (above == prefix[t]) atomicAdd(&h[t][digit], 1u);
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kScoreTargets * bins; i += blockDim.x) {
-        const uint32_t t = i / bins, bin = i % bins;
+        const uint32_t t = i >> width, bin = i & (bins - 1u);
         if (h[t][bin]) atomicAdd(hist + (size_t(c) * kScoreTargets + t) * kScoreHistBins + bin, h[t][bin]);
     }
 }
@@ -214,7 +226,7 @@ __global__ void __launch_bounds__(256) select_hist_kernel(const float* __restric
 __global__ void __launch_bounds__(256) select_pick_kernel(ScoreState* __restrict__ state, uint32_t first,
                                                           uint32_t width, uint32_t* __restrict__ hist) {
     constexpr uint32_t kPer = kScoreHistBins / 256u;
-    __shared__ uint64_t warp_total[8];
+    __shared__ uint64_t warp_total[kScoreTargets][8];
     ScoreState& S = state[blockIdx.x];
     const uint64_t count = S.count;
     if (count == 0u) return;
@@ -228,40 +240,55 @@ __global__ void __launch_bounds__(256) select_pick_kernel(ScoreState* __restrict
         prefix[t] = S.prefix[t];
         rank[t] = first ? uint64_t(floor(double(count - 1u) * quantile[t] + 0.5)) : S.rank[t];
     }
-    __syncthreads();  // all read before one of them writes
-    uint32_t own[kPer] = {};
-    uint64_t before = 0u;
+    // all rows' loads under way at once, 16 bytes each
+    uint32_t own[kScoreTargets][kPer];
+    uint64_t upto[kScoreTargets];
+    uint32_t owner = 0u;  // the prefixes ascend with the targets' ranks: equal ones are neighbours
+    static_assert(kPer == 8u, "two 16-byte words of bins per thread");
+    uint4* const rows = reinterpret_cast<uint4*>(hist + size_t(blockIdx.x) * kScoreTargets * kScoreHistBins) + tid * 2u;
 #pragma unroll
     for (uint32_t t = 0; t < kScoreTargets; ++t) {
-        // the prefixes ascend with the targets' ranks: equal ones are neighbours
-        if (first ? t == 0u : t == 0u || prefix[t] != prefix[t - 1u]) {
-            uint32_t* row = hist + (size_t(blockIdx.x) * kScoreTargets + t) * kScoreHistBins + tid * kPer;
-            uint64_t mine = 0u;
+        if (t && !first && prefix[t] != prefix[t - 1u]) owner = t;
 #pragma unroll
-            for (uint32_t i = 0; i < kPer; ++i) {
-                own[i] = row[i];
-                row[i] = 0u;
-                mine += own[i];
-            }
-            uint64_t upto = mine;
-#pragma unroll
-            for (uint32_t o = 1; o < 32u; o <<= 1) {
-                const uint64_t v = __shfl_up_sync(0xffffffffu, upto, o);
-                if (lane >= o) upto += v;
-            }
-            if (lane == 31u) warp_total[warp] = upto;
-            __syncthreads();
-            before = upto - mine;
-            for (uint32_t w = 0; w < warp; ++w) before += warp_total[w];
-            __syncthreads();
+        for (uint32_t q = 0; q < 2u; ++q) {
+            const uint4 v = rows[owner * (kScoreHistBins / 4u) + q];
+            own[t][q * 4u] = v.x;
+            own[t][q * 4u + 1u] = v.y;
+            own[t][q * 4u + 2u] = v.z;
+            own[t][q * 4u + 3u] = v.w;
         }
-        uint64_t below = before;
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < kScoreTargets; ++t) {
+        upto[t] = 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; ++i) upto[t] += own[t][i];
+        // this thread's bins, which it has read
+        rows[t * (kScoreHistBins / 4u)] = rows[t * (kScoreHistBins / 4u) + 1u] = make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < kScoreTargets; ++t) {
+        const uint64_t mine = upto[t];
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint64_t v = __shfl_up_sync(0xffffffffu, upto[t], o);
+            if (lane >= o) upto[t] += v;
+        }
+        if (lane == 31u) warp_total[t][warp] = upto[t];
+        upto[t] -= mine;
+    }
+    __syncthreads();  // and the state is read by all before one of them writes it
+#pragma unroll
+    for (uint32_t t = 0; t < kScoreTargets; ++t) {
+        uint64_t below = upto[t];
+        for (uint32_t w = 0; w < warp; ++w) below += warp_total[t][w];
+#pragma unroll
         for (uint32_t i = 0; i < kPer; ++i) {
-            if (rank[t] >= below && rank[t] - below < own[i]) {  // one thread has it
+            if (rank[t] >= below && rank[t] - below < own[t][i]) {  // one thread has it
                 S.rank[t] = rank[t] - below;
                 S.prefix[t] = (prefix[t] << width) | (tid * kPer + i);
             }
-            below += own[i];
+            below += own[t][i];
         }
     }
 }
@@ -287,19 +314,27 @@ __global__ void __launch_bounds__(256) scale_select_kernel(const double* __restr
                                                            uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kScoreHistBins];
     __shared__ uint32_t last;
+    __shared__ uint64_t warp_total[8];
     const uint32_t bins = 1u << width, top = shift + width;
     for (uint32_t i = threadIdx.x; i < bins; i += blockDim.x) h[i] = 0u;
     const uint64_t prefix = first ? 0u : state->prefix;
     __syncthreads();
     uint32_t n = 0u;
-    for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < samples;
-         s += uint64_t(gridDim.x) * blockDim.x) {
-        const double y = ref_xyz[s * 3 + 1];
-        if (!isfinite(y)) continue;
-        const uint64_t key = order_key(y);
-        if (!first && (key >> top) != prefix) continue;
-        ++n;
-        atomicAdd(&h[uint32_t(key >> shift) & (bins - 1u)], 1u);
+    for (uint64_t tile = uint64_t(blockIdx.x) * kTile; tile < samples; tile += uint64_t(gridDim.x) * kTile) {
+        double y[kSamples];
+#pragma unroll
+        for (uint32_t j = 0; j < kSamples; ++j) {
+            const uint64_t s = tile + j * 256u + threadIdx.x;
+            y[j] = s < samples ? ref_xyz[s * 3 + 1] : CUDART_INF;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kSamples; ++j) {
+            if (!isfinite(y[j])) continue;
+            const uint64_t key = order_key(y[j]);
+            if (!first && (key >> top) != prefix) continue;
+            ++n;
+            atomicAdd(&h[uint32_t(key >> shift) & (bins - 1u)], 1u);
+        }
     }
     n = __reduce_add_sync(0xffffffffu, n);
     if (first && (threadIdx.x & 31u) == 0u && n)
@@ -313,28 +348,37 @@ __global__ void __launch_bounds__(256) scale_select_kernel(const double* __restr
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x < 32u) {  // one warp scans the digit's histogram, 32 bins at a time
-        const uint64_t count = *reinterpret_cast<volatile uint64_t*>(&state->count);
-        uint64_t rank = first ? (count ? uint64_t(floor(double(count - 1u) * 0.99 + 0.5)) : 0u) : state->rank;
-        uint64_t below = 0u;
-        for (uint32_t b = 0u; b < bins; b += 32u) {
-            const uint32_t mine = *reinterpret_cast<volatile uint32_t*>(hist + b + threadIdx.x);
-            hist[b + threadIdx.x] = 0u;
-            uint64_t upto = mine;
-#pragma unroll
-            for (uint32_t o = 1; o < 32u; o <<= 1) {
-                const uint64_t v = __shfl_up_sync(0xffffffffu, upto, o);
-                if (threadIdx.x >= o) upto += v;
-            }
-            const uint64_t before = below + upto - mine;
-            if (rank >= before && rank - before < mine) {  // one lane has it
-                state->prefix = (prefix << width) | (b + threadIdx.x);
-                state->rank = rank - before;
-            }
-            below += __shfl_sync(0xffffffffu, upto, 31);
-        }
-        if (threadIdx.x == 0u) state->ended = 0u;
+    // a block scan of the digit's histogram, bins / 256 neighbouring bins to a thread
+    // (32 bins at a time by one warp: 28 of a pass's 45 us)
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, per = bins / 256u;
+    const uint64_t count = *reinterpret_cast<volatile uint64_t*>(&state->count);
+    const uint64_t rank = first ? (count ? uint64_t(floor(double(count - 1u) * 0.99 + 0.5)) : 0u) : state->rank;
+    for (uint32_t i = tid; i < bins; i += 256u) {
+        h[i] = *reinterpret_cast<volatile uint32_t*>(hist + i);
+        hist[i] = 0u;
     }
+    __syncthreads();
+    uint64_t mine = 0u;
+    for (uint32_t i = 0; i < per; ++i) mine += h[tid * per + i];
+    uint64_t upto = mine;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint64_t v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+    }
+    if (lane == 31u) warp_total[warp] = upto;
+    __syncthreads();  // the rank is read by all before one of them writes it
+    uint64_t below = upto - mine;
+    for (uint32_t w = 0; w < warp; ++w) below += warp_total[w];
+    for (uint32_t i = 0; i < per; ++i) {
+        const uint32_t own = h[tid * per + i];
+        if (rank >= below && rank - below < own) {  // one thread has it
+            state->prefix = (prefix << width) | (tid * per + i);
+            state->rank = rank - below;
+        }
+        below += own;
+    }
+    if (tid == 0u) state->ended = 0u;
 }
 
 // The scale: the selected Y, at least 1e-12 (also without a finite one).
@@ -395,8 +439,8 @@ cudaError_t launch_score(const ScoreLaunch& w, cudaStream_t stream) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint32_t shift[3] = {21u, 10u, 0u}, width[3] = {11u, 11u, 10u};
-    const uint32_t readers = uint32_t(
-        std::min<uint64_t>((w.samples + 1023u) / 1024u, std::max(1u, 8u * w.sms / w.combos)));
+    const uint32_t readers = uint32_t(  // five blocks of 40 KB a SM, in one wave
+        std::min<uint64_t>(tiles, std::max(1u, 5u * w.sms / w.combos)));
     for (int pass = 0; pass < 3; ++pass) {
         if (pass > 0) {
             select_hist_kernel<<<dim3(readers, w.combos), 256, 0, stream>>>(w.dist, w.samples, w.state, shift[pass],

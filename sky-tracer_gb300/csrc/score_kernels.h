@@ -8,6 +8,7 @@
 namespace sky {
 
 constexpr uint32_t kScoreHistBins = 2048;  // widest radix-selection pass: 11 bits
+constexpr uint32_t kScoreGroup = 4;        // combinations of a block of the distances
 constexpr uint32_t kScoreTargets = 5;      // p50, p90, p95, p99, max
 
 // One combination's sums over its finite distances, and the selection of its

@@ -1295,8 +1295,10 @@ extern "C" int sky_cuda_score_combos(const float* bands, uint32_t band_count, ui
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
     // combinations per launch sequence: as many as keep their distances (64 MB) in the L2 cache
     // until they are selected from, one at least
-    const uint32_t chunk = uint32_t(
+    uint32_t chunk = uint32_t(
         std::max<uint64_t>(1, std::min<uint64_t>({combo_count, 1024u, (uint64_t(1) << 24) / samples})));
+    // whole groups of the distances' blocks (25 of 655 360 samples would leave the seventh three quarters empty)
+    if (chunk < combo_count && chunk > kScoreGroup) chunk -= chunk % kScoreGroup;
     // one allocation: the combinations, their states (all of them), one chunk's histograms and distances
     size_t off = 0;
     auto reserve = [&off](size_t bytes) {
