@@ -150,8 +150,8 @@ typedef enum SkyKernel {
     SKY_KERNEL_AUTO = 0,       /* the wavefront kernel                                   */
     SKY_KERNEL_PLAIN = 1,      /* one chain per lane, a warp per cell; cell sums in a
                                   fixed order                                            */
-    SKY_KERNEL_WAVEFRONT = 2   /* persistent ray loop: one ray per lane per iteration,
-                                  per-lane chain regeneration                            */
+    SKY_KERNEL_WAVEFRONT = 2   /* persistent: a warp runs one stage of 32 paths at a time;
+                                  small renders, a ray loop with a path per lane         */
 } SkyKernel;
 
 /* Add into the sums already held by the outputs instead of overwriting them

@@ -3,7 +3,7 @@
 The reference dispatches a fixed 8x8x1 workgroup per (pixel block, band) and
 two samples per dispatch (integrator.rs:254-283); nothing is tuned.  Here the
 shape of the wavefront kernel is a per-scene setting (SkyTuning): the
-resident blocks per SM it is compiled for (registers per lane against lanes
+warps per block it is compiled for (registers per lane against lanes
 in flight) and the crossing cost that sets how far the tracking grid is
 merged.  `autotune` times each candidate on a reduced-sample probe of the
 caller's own render (same image, same scene, fewer samples per pixel) with
