@@ -16,11 +16,11 @@
 // What bounds it: instruction issue, as the tracer.  The ray loop runs all event
 // code once per ray: 8 to 10 of 32 lanes active.  16.8 M chains (128x64, 32 bands,
 // 64 spp): primal 3.79 -> 2.18 ms, gradient with the primal's chain radiance 4.05 ->
-// 3.09 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.1 ms and
+// 3.00 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.1 ms and
 // 29.7 -> 20.2 ms.  The primal issues at 83 % with 24 lanes active; the gradient at
 // 52 % with 17: its code is still more than the instruction caches hold ("no
 // instruction" 3.0 cycles per issue), and its layer gradients are shared-memory
-// atomics (short scoreboard 2.3).
+// atomics (short scoreboard 2.3, with one copy a warp).
 
 #include <algorithm>
 

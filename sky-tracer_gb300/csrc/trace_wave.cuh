@@ -26,7 +26,7 @@
 // ray loop (trace_ray.cuh) keeps each lane's path in registers and runs all event
 // code once per ray: 9.5 of 32 lanes active per instruction, 7.9 G warp
 // instructions and 7.42 ms for 42 M chains (128x64, 81 bands, 64 spp).  Here
-// 21 lanes are active, for 5.1 G instructions at 87 % of the issue slots and 4.65
+// 22.6 lanes are active, for 4.9 G instructions at 86 % of the issue slots and 4.65
 // ms; what is left is the rays' different lengths (tracking is two fifths) and
 // the queues (a fifth).  What took it there: tracking right after the stage,
 // instead of queueing every ray for it, 6.2 to 5.4 ms; staying with a stage, 5.15
