@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
     n.clear();
     bool watchdog = false;
     uint32_t idle = 0u, turn = (threadIdx.x >> 5) & 3u;
+    uint32_t job_hint = 0u;  // the job of the last chains that the warp took: chains are taken in order
 
     for (uint32_t batch = 0u;;) {
         uint32_t stage, take, id;
@@ -544,16 +545,21 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocksPerSm)
             base = __shfl_sync(kFull, base, 0);
             const unsigned long long at = base + lane;
             const bool more = on && at < total_chains;
-            if (more) {
-                uint32_t job = 0u;
-                if constexpr (!kSingle) {  // the last job whose first chain is <= at
-                    uint32_t hi = num_jobs;
-                    while (hi - job > 1u) {
-                        const uint32_t mid = (job + hi) >> 1;
-                        if (__ldg(&jobs[mid].chain_begin) <= at) job = mid;
-                        else hi = mid;
-                    }
+            uint32_t job = job_hint;
+            if (!kSingle && more) {
+                // the last job whose first chain is <= at: mostly that of the warp's last chains
+                // (searching all jobs each time: 16 images of 128x64, 40 bands, 130.5
+                // against 126.9 ms)
+                uint32_t hi = num_jobs;
+                if (job + 1u < hi && __ldg(&jobs[job + 1u].chain_begin) > at) hi = job + 1u;
+                while (hi - job > 1u) {
+                    const uint32_t mid = (job + hi) >> 1;
+                    if (__ldg(&jobs[mid].chain_begin) <= at) job = mid;
+                    else hi = mid;
                 }
+            }
+            if (!kSingle) job_hint = __shfl_sync(kFull, job, 0);
+            if (more) {
                 const DevLaunch& JL = job_launch<kSingle>(L0, jobs, job);
                 const unsigned long long rel = kSingle ? at : at - __ldg(&jobs[job].chain_begin);
                 // cell and sample, band and pixel of the slab, row and column: quotients by products

@@ -98,6 +98,27 @@ def test_jobs_of_unequal_size_share_the_queues(gpu, dome_scene):
             _same([x.cpu().numpy() for x in b], want, c.spp + 8)
 
 
+@pytest.mark.parametrize("large", [0, 20, 39])
+def test_many_jobs_smaller_than_a_batch(gpu, dome_scene, large):
+    """One job of most chains among 39 of a few each, which a warp's 32 chains span: the lookup
+    that starts from the job of the warp's last chains."""
+    import torch
+    stream = torch.cuda.current_stream().cuda_stream
+    base = dict(phase_sampling=_abi.PHASE_TABULATED, tracking=MERGED)
+    with GpuScene(dome_scene) as gs:
+        cfgs = [RenderConfig(width=1, height=1, spp=1 + i % 3, seed=i, **base) for i in range(40)]
+        cfgs[large] = RenderConfig(width=24, height=12, spp=_samples(24 * 12 * gs.band_count, MERGED), seed=5, **base)
+        bufs = [_buffers(c.pixels * gs.band_count) for c in cfgs]
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        gs.render_batch([(c, None, {"cell_sum": b[0].data_ptr(), "cell_sumsq": b[1].data_ptr(),
+                                    "status": st.data_ptr()}) for c, b in zip(cfgs, bufs)], stream)
+        torch.cuda.synchronize()
+        assert int(st.item()) == 0
+        for c, b in zip(cfgs, bufs):
+            _same([x.cpu().numpy() for x in b], _sums(gs, RenderConfig(**{**c.__dict__, "kernel": _abi.KERNEL_PLAIN})),
+                  c.spp)
+
+
 def test_iteration_limit_stops_the_queues(gpu, dome_scene):
     spp = _samples(16 * 8 * dome_scene.band_count, MERGED)
     cfg = RenderConfig(width=16, height=8, spp=spp, phase_sampling=_abi.PHASE_TABULATED, tracking=MERGED)
