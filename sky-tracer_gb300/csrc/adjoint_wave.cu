@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "adjoint_device.cuh"
+#include "launch_limits.h"
 #include "stage_queues.cuh"
 
 namespace sky {
@@ -744,9 +745,7 @@ cudaError_t launch_shape(const AdjCtx& A, const AdjJobs& J, double* layer_grad, 
         while (paths > 32u && !fits(paths, 1)) paths -= 32u;
     }
     const size_t smem = bytes(paths);
-    if (smem > 48u * 1024u &&
-        (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
-        return e;
+    if ((e = allow_shared_memory(k, smem)) != cudaSuccess) return e;
     const size_t need = size_t(fits(paths, 2) ? 2 : 1) * (smem + size_t(reserved));
     const int pct = int(std::min<size_t>(100u, (need * 100u + size_t(smem_sm) - 1u) / size_t(smem_sm)));
     if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, std::max(pct, 1)) != cudaSuccess)

@@ -43,6 +43,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "launch_limits.h"
 #include "mie_kernels.h"
 
 namespace sky {
@@ -275,10 +276,7 @@ cudaError_t launch_mie_bake(const MieItem* items, uint32_t bands, uint32_t radii
     mie_coefficients_kernel<<<(count + 3u) / 4u, 128, 0, stream>>>(items, bands, radii, dscratch, riccati, ab, q);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t smem = size_t(max_terms) * sizeof(float4);
-    if (smem > 48u * 1024u) {
-        e = cudaFuncSetAttribute(mie_angles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return e;
-    }
+    if ((e = allow_shared_memory(reinterpret_cast<const void*>(mie_angles_kernel), smem)) != cudaSuccess) return e;
     // four blocks per SM: the radii of a band in shares that each hold large and small ones
     const uint32_t tiles = uint32_t((uint64_t(bins) + kAngleThreads * kAngleBins - 1u) / (kAngleThreads * kAngleBins));
     const uint64_t each = uint64_t(bands) * tiles;

@@ -35,6 +35,7 @@
 
 #include <algorithm>
 
+#include "launch_limits.h"
 #include "trace_common.cuh"
 
 namespace sky {
@@ -423,9 +424,7 @@ cudaError_t launch_ray_shape(const WaveLaunch& w, cudaStream_t stream) {
     // aerosol species; the largest scenes the library accepts (1024 knots, 256 bands) need 77 KB,
     // beyond the 48 KB a launch gets without opting in
     const size_t smem = ray_smem_bytes(w.scene.knot_count, w.scene.band_count, uint32_t(kAer));
-    if (smem > 48u * 1024u &&
-        (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
-        return e;
+    if ((e = allow_shared_memory(k, smem)) != cudaSuccess) return e;
     // Prefer the smallest shared-memory carveout that holds kMinBlocks blocks' tables: the
     // rest of the SM's L1/shared array caches the phase tables, extinction rows and merged
     // grid (the largest carveout costs 6 % on the production render).  A hint: if the

@@ -48,6 +48,7 @@
 
 #include <algorithm>
 
+#include "launch_limits.h"
 #include "stage_queues.cuh"
 #include "trace_common.cuh"
 
@@ -691,9 +692,7 @@ cudaError_t launch_wave_shape(const WaveLaunch& w, cudaStream_t stream) {
         while (paths > 32u && !fits(paths, 1)) paths -= 32u;
     }
     const size_t smem = wave_smem_bytes<kAer>(w.scene.knot_count, w.scene.band_count, paths);
-    if (smem > 48u * 1024u &&
-        (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
-        return e;
+    if ((e = allow_shared_memory(k, smem)) != cudaSuccess) return e;
     // Prefer the smallest shared-memory carveout that holds two blocks: the rest of the
     // SM's L1/shared array caches the phase tables, extinction rows and merged grid.  A
     // hint: if the driver refuses it, the launch goes ahead with its own choice.
