@@ -11,7 +11,8 @@
 // the ray's end is taken up by its next stage, those of the vertices where they
 // are made; band gradients stay in the lane's registers while its band does, the
 // Mie albedo's and g's for the whole kernel, and layer gradients go to the warp's
-// copy in shared memory.
+// copy in shared memory, from which the warp moves them to the FP64 outputs every
+// kFlushBatches of its batches.
 //
 // What bounds it: instruction issue, as the tracer.  The ray loop runs all event
 // code once per ray: 8 to 10 of 32 lanes active.  16.8 M chains (128x64, 32 bands,
@@ -57,6 +58,18 @@ enum : uint32_t { kFlagShadow = 1u << 8, kFlagGround = 1u << 9, kFlagTop = 1u <<
 
 // Rays left to the track queue, and crossings left to the next step, as in the tracer.
 constexpr uint32_t kPark = 14, kCrossing = 3;
+
+// Batches of a warp between two moves of its layer-gradient copies to the FP64
+// gradient, the block's warps in turn.  An FP32 copy's rounding error grows with the
+// terms that it takes between them: a copy of the block's as many as a copy of one
+// warp's, both fewer than a warp's copy in the ray loop takes of the smallest launch that
+// comes here.  Largest error of 54.8 M chains, relative to the largest gradient, without
+// the moves, with them and in the ray loop: 114 layers (one copy per block) 3.1e-4,
+// 1.9e-7 and 1.5e-5; 100 layers (one per warp) 1.0e-5, 3.5e-7 and 8.8e-6.  (256 batches:
+// 4.3e-7 and 1.5e-6, and at 300 layers 14.2 M chains still 3 times the ray loop's.)  The
+// moves cost 16.8 M chains of 64 layers 1.3 %, 54.8 M of 1000 layers 4.7 %, the fit's 67 M,
+// without a layer gradient, nothing.
+constexpr uint32_t kFlushBatches = 64;
 
 // A path in shared memory, rows of 16 bytes: A-F as the tracer's, then
 //   G  the vertex: unscaled Rayleigh, Mie and ozone coefficients, layer
@@ -232,7 +245,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float* const grads = reinterpret_cast<float*>(
         smem + align16(size_t(paths) * kRows * 16u + sizeof(Queues) + size_t(kQueues) * queue_slots(paths) * 2u));
-    float* const sg = kGrad && copies ? grads + (warp * 2u + (lane & 1u)) % copies * nlayer : nullptr;
+    // two copies per warp (of its even and its odd lanes), one, or one per block
+    const bool two = copies == 2u * kWarps;
+    float* const sg = kGrad && copies ? grads + (two ? warp * 2u + (lane & 1u) : warp % copies) * nlayer : nullptr;
     float* const sb = grads + copies * nlayer;
     for (uint32_t i = threadIdx.x; i < used_paths; i += blockDim.x)
         pool[i * kRows + kB] = make_float4(0.0f, as_f(kFresh), 0.0f, 0.0f);
@@ -250,6 +265,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
         const Taken taken = queues.take(lane, turn, idle, batch, 0xffffffffu, status, stage, take, id);
         if (taken == kOutOfWork) break;
         if (taken == kNothing) continue;
+        if (kGrad && copies && batch % kFlushBatches == warp * (kFlushBatches / uint32_t(kWarps))) {
+            float* const own = grads + (two ? warp * 2u : warp % copies) * nlayer;
+#pragma unroll 1
+            for (uint32_t i = lane; i < nlayer; i += 32u) {
+                double v = double(atomicExch(own + i, 0.0f));
+                if (two) v += double(atomicExch(own + nlayer + i, 0.0f));
+                if (v != 0.0) atomicAdd(layer_grad + i, v);
+            }
+        }
         const bool on = lane < take;
         float4* const P = pool + id * kRows;
         uint32_t next = kQNone;
@@ -697,9 +721,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; layer_grad && i < nlayer; i += blockDim.x) {
-        float v = 0.0f;
-        for (uint32_t k = 0; k < copies; ++k) v += grads[k * nlayer + i];
-        if (v != 0.0f) atomicAdd(layer_grad + i, double(v));
+        double v = 0.0;
+        for (uint32_t k = 0; k < copies; ++k) v += double(grads[k * nlayer + i]);
+        if (v != 0.0) atomicAdd(layer_grad + i, v);
     }
     if (band_grad)
         for (uint32_t i = threadIdx.x; i < kAdjBandParams * bands; i += blockDim.x)
