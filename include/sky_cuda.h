@@ -257,8 +257,7 @@ typedef struct SkyDeviceOutputs {
  */
 typedef struct SkyTuning {
     uint32_t variant;            /* warps per SM the kernel is compiled for: 0 = 24 (80 registers
-                                    per lane), 1 = 16 (128), 2 = 32 (64); renders of few chains
-                                    per lane always run the last                                */
+                                    per lane), 1 = 16 (128), 2 = 32 (64)                        */
     uint32_t max_blocks_per_sm;  /* 0 = occupancy limit                                          */
     uint32_t all_species;        /* 1 = the kernels evaluate all four aerosol species; 0 = only
                                     species 0 when species 1-3 carry no aerosol anywhere in the

@@ -24,7 +24,9 @@ cudaError_t launch_trace_plain(const DevScene& S, const DevLaunch& L, double* ce
 
 // Persistent wavefront tracer (trace_wave.cu): stage queues over a pool of paths per block,
 // over a job table.
-constexpr uint32_t kWaveVariants = 3;  // warps per block (two blocks per SM): variant 0 -> 12, 1 -> 8, 2 -> 16
+// Kernel shapes (SkyTuning.variant).  Stage queues: warps per block (two blocks per SM),
+// variant 0 -> 12, 1 -> 8, 2 -> 16; ray loop: blocks of 8 warps per SM, 0 -> 3, 1 -> 2, 2 -> 4.
+constexpr uint32_t kWaveVariants = 3;
 
 struct WaveLaunch {
     DevScene scene;                // the first job's scene: its tables and constants are every job's

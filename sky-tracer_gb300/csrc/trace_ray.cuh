@@ -49,7 +49,6 @@ using wave::stage_medium;
 using wave::staged_medium_bytes;
 
 constexpr uint32_t kWaveThreads = 256;
-constexpr int kMinBlocks = 4;  // resident blocks per SM: 64 registers per lane
 constexpr uint32_t kNoCell = 0xffffffffu;
 
 // What a lane does next.
@@ -116,7 +115,11 @@ __host__ __device__ inline size_t ray_smem_bytes(uint32_t knots, uint32_t bands,
 // they would hold are worth ~5 % at 64 registers per lane).
 // kAer: aerosol species evaluated by the medium functions (1 or kSpecies,
 // coefficients_at()).
-template <int kTracking, int kPhase, bool kSingle, bool kCount, int kAer>
+// kMinBlocks: resident blocks per SM that the registers leave room for
+// (SkyTuning.variant: 4, 3 or 2 blocks of 64, 80 or 128 registers per lane).  Four are
+// the fastest while the medium's tables are small; of tables that fill the SM with three
+// blocks, three: 41 bands, 1000 layers, 2.0 M chains 0.53 against 0.46 ms.
+template <int kTracking, int kPhase, int kMinBlocks, bool kSingle, bool kCount, int kAer>
 __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     ray_kernel(const __grid_constant__ DevScene S, const __grid_constant__ DevLaunch L0,
                 const DevJob* __restrict__ jobs, uint32_t num_jobs,
@@ -413,10 +416,10 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     if (__any_sync(kFull, watchdog) && lane == 0u) atomicOr(status, 1u);
 }
 
-template <int kTracking, int kPhase, bool kSingle, bool kCount, int kAer>
+template <int kTracking, int kPhase, int kMinBlocks, bool kSingle, bool kCount, int kAer>
 cudaError_t launch_ray_shape(const WaveLaunch& w, cudaStream_t stream) {
     const void* k =
-        reinterpret_cast<const void*>(ray_kernel<kTracking, kPhase, kSingle, kCount, kAer>);
+        reinterpret_cast<const void*>(ray_kernel<kTracking, kPhase, kMinBlocks, kSingle, kCount, kAer>);
     int dev = 0, per_sm = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -446,19 +449,29 @@ cudaError_t launch_ray_shape(const WaveLaunch& w, cudaStream_t stream) {
     // a warp per cell at most
     const uint64_t want = (uint64_t(w.total_cells) * 32u + kWaveThreads - 1u) / kWaveThreads;
     const uint32_t blocks = uint32_t(std::max<uint64_t>(1u, std::min<uint64_t>(uint64_t(per_sm) * uint64_t(w.sms), want)));
-    ray_kernel<kTracking, kPhase, kSingle, kCount, kAer><<<blocks, kWaveThreads, smem, stream>>>(
+    ray_kernel<kTracking, kPhase, kMinBlocks, kSingle, kCount, kAer><<<blocks, kWaveThreads, smem, stream>>>(
         w.scene, w.launch0, w.jobs, w.num_jobs, w.total_cells, reinterpret_cast<uint32_t*>(w.work_counter), w.counters, w.status,
         w.iteration_limit ? w.iteration_limit : kMaxIterations);
     return cudaGetLastError();
 }
 
+template <int kTracking, int kPhase, bool kSingle, bool kCount, int kAer>
+cudaError_t launch_ray_variant(const WaveLaunch& w, cudaStream_t stream) {
+    switch (w.variant) {
+        case 0: return launch_ray_shape<kTracking, kPhase, 3, kSingle, kCount, kAer>(w, stream);
+        case 1: return launch_ray_shape<kTracking, kPhase, 2, kSingle, kCount, kAer>(w, stream);
+        case 2: return launch_ray_shape<kTracking, kPhase, 4, kSingle, kCount, kAer>(w, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 template <int kTracking, int kPhase, int kAer>
 cudaError_t launch_ray_species(const WaveLaunch& w, cudaStream_t stream) {
     if (w.num_jobs == 1u)
-        return w.counters ? launch_ray_shape<kTracking, kPhase, true, true, kAer>(w, stream)
-                          : launch_ray_shape<kTracking, kPhase, true, false, kAer>(w, stream);
-    return w.counters ? launch_ray_shape<kTracking, kPhase, false, true, kAer>(w, stream)
-                      : launch_ray_shape<kTracking, kPhase, false, false, kAer>(w, stream);
+        return w.counters ? launch_ray_variant<kTracking, kPhase, true, true, kAer>(w, stream)
+                          : launch_ray_variant<kTracking, kPhase, true, false, kAer>(w, stream);
+    return w.counters ? launch_ray_variant<kTracking, kPhase, false, true, kAer>(w, stream)
+                      : launch_ray_variant<kTracking, kPhase, false, false, kAer>(w, stream);
 }
 
 template <int kTracking, int kPhase>
