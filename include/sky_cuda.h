@@ -322,6 +322,9 @@ void sky_cuda_scene_destroy(SkyScene* scene);
  * from the scene's majorant grid.  No counterpart in the reference. */
 int sky_cuda_scene_set_tuning(SkyScene* scene, const SkyTuning* tuning);
 int sky_cuda_scene_get_tuning(const SkyScene* scene, SkyTuning* tuning);
+/* Chains (pixels x bands x samples of a launch) from which the wavefront tracer runs its stage
+ * queues in this tracking mode, and below which its ray loop: two kernels, whose best shapes differ. */
+int sky_cuda_queue_chains(const SkyScene* scene, uint32_t tracking, uint64_t* chains);
 
 /*
  * Render the spectral film into host memory: `film_out` receives

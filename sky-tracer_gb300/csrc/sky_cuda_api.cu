@@ -503,6 +503,15 @@ int sky_cuda_scene_get_tuning(const SkyScene* s, SkyTuning* t) {
     return SKY_OK;
 }
 
+int sky_cuda_queue_chains(const SkyScene* s, uint32_t tracking, uint64_t* chains) {
+    if (!s || !chains) return set_error(SKY_ERR_INVALID_CONFIG, "scene and chains must not be null");
+    if (tracking > SKY_TRACKING_MERGED_LAYERS) return set_error(SKY_ERR_INVALID_CONFIG, "unknown tracking mode");
+    int sms = 0;
+    const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    if (e != cudaSuccess) return cuda_fail(SKY_ERR_NO_DEVICE, "counting SMs", e);
+    *chains = wave_queue_chains(tracking, aerosol_species(s->dev, s->tuning.all_species != 0u), sms);
+    return SKY_OK;
+}
 
 const char* sky_cuda_version(void) { return "sky_cuda 0.1.0 (abi 1, sm_103a)"; }
 

@@ -52,6 +52,8 @@ struct WaveLaunch {
 // the jobs' cell sums (zeroed first unless a job accumulates), film, XYZ,
 // XYZ variance and linear sRGB.
 cudaError_t launch_trace_wave(const WaveLaunch& w, cudaStream_t stream);
+// Chains from which a launch takes the stage queues; the ray loop traces smaller ones.
+uint64_t wave_queue_chains(uint32_t tracking, uint32_t aerosol_species, int sms);
 // The tracing kernels alone, per tracking mode: the ray loop of small renders
 // (trace_ray_*.cu) and the stage queues (trace_wave_*.cu).
 cudaError_t launch_ray_segment_restart(const WaveLaunch& w, cudaStream_t stream);

@@ -27,23 +27,23 @@ __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restr
     }
 }
 
-// Whether a launch goes to the ray loop (trace_ray.cuh) rather than to the stage
-// queues (trace_wave.cuh): where it has so few chains per lane of the chip
+}  // namespace
+
+// A launch goes to the ray loop (trace_ray.cuh) rather than to the stage
+// queues (trace_wave.cuh) where it has so few chains per lane of the chip
 // (1024 lanes per SM) that its longest chains decide its time.  Measured with
 // both kernels (ms, ray loop against queues):
 //   merged layers      one species: 3.1 M chains 0.63 / 0.65, 4.2 M 0.79 / 0.75: 24 per lane;
 //                      four: 4.0 M 1.47 / 1.60, 5.4 M 1.86 / 1.81: 34 per lane
 //   residual carry     131 k 0.52 / 0.68, 262 k 0.63 / 0.62, 524 k 0.82 / 0.70: 2 per lane
 //   segment restart    0.67 M 1.25 / 1.34, 1.0 M 1.63 / 1.12: 5 per lane
-bool small_render(const WaveLaunch& w) {
-    const uint64_t per_lane = w.tracking == SKY_TRACKING_SEGMENT_RESTART  ? 5u
-                              : w.tracking == SKY_TRACKING_RESIDUAL_CARRY ? 2u
-                              : w.aerosol_species == 1u                   ? 24u
-                                                                          : 34u;
-    return w.total_chains < per_lane * 1024u * uint64_t(w.sms);
+uint64_t wave_queue_chains(uint32_t tracking, uint32_t aerosol_species, int sms) {
+    const uint64_t per_lane = tracking == SKY_TRACKING_SEGMENT_RESTART  ? 5u
+                              : tracking == SKY_TRACKING_RESIDUAL_CARRY ? 2u
+                              : aerosol_species == 1u                   ? 24u
+                                                                        : 34u;
+    return per_lane * 1024u * uint64_t(sms);
 }
-
-}  // namespace
 
 cudaError_t launch_trace_wave(const WaveLaunch& asked, cudaStream_t stream) {
     WaveLaunch w = asked;
@@ -57,7 +57,7 @@ cudaError_t launch_trace_wave(const WaveLaunch& asked, cudaStream_t stream) {
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&w.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    const bool small = small_render(w);
+    const bool small = w.total_chains < wave_queue_chains(w.tracking, w.aerosol_species, w.sms);
     switch (w.tracking) {
         case SKY_TRACKING_SEGMENT_RESTART:
             e = small ? launch_ray_segment_restart(w, stream) : launch_wave_segment_restart(w, stream);

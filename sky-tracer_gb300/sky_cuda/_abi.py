@@ -171,6 +171,7 @@ _SIGNATURES = {
     "sky_cuda_scene_destroy": (None, [_vp]),
     "sky_cuda_scene_set_tuning": (ctypes.c_int, [_vp, ctypes.POINTER(SkyTuning)]),
     "sky_cuda_scene_get_tuning": (ctypes.c_int, [_vp, ctypes.POINTER(SkyTuning)]),
+    "sky_cuda_queue_chains": (ctypes.c_int, [_vp, ctypes.c_uint32, ctypes.POINTER(ctypes.c_uint64)]),
     "sky_cuda_render": (ctypes.c_int, [_vp, ctypes.POINTER(SkyRenderConfig), _fp, ctypes.c_size_t,
                                        ctypes.POINTER(SkyRenderStats)]),
     "sky_cuda_render_xyz": (ctypes.c_int, [_vp, ctypes.POINTER(SkyRenderConfig), _fp, ctypes.c_size_t,

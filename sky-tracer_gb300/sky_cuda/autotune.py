@@ -44,18 +44,28 @@ def _time_render(gs: GpuScene, cfg: RenderConfig, repeats: int) -> float:
     return best
 
 
+def _probe_spp(gs: GpuScene, config: RenderConfig) -> int:
+    """Samples of a probe that runs the kernel of the render itself: enough for the stage queues
+    where the render has them (a scene that does not say where its queues begin has one kernel)."""
+    spp = min(config.spp, max(64, config.spp // 8))
+    line = gs.queue_spp(config) if hasattr(gs, "queue_spp") else 0
+    return max(spp, line) if config.spp >= line else spp
+
+
 def autotune(gs: GpuScene, config: RenderConfig, space: dict | None = None, probe_spp: int | None = None,
              repeats: int = 2, apply: bool = True):
     """Time every combination of `space` on a probe render and keep the best.
 
     Returns (best_tuning_dict, [(tuning_dict, ms), ...]).  The probe renders
     the caller's full image at `probe_spp` samples (default: spp/8, at least 64
-    or the whole render: below two warps' worth of samples per cell the lanes
-    of a warp sit idle in a way the render itself does not, and a 64x32 render
-    probed at 8 spp picked a shape 24 % slower at its 64 spp).
+    or the whole render: with few samples per cell the ray loop's lanes sit idle
+    in a way the render itself does not, and a 64x32 render probed at 8 spp picked
+    a shape 24 % slower at its 64 spp).  A render that takes the stage queues is
+    probed with as many samples as take the probe there too: the two kernels'
+    best shapes differ.
     """
     space = dict(DEFAULT_SPACE if space is None else space)
-    probe = replace(config, spp=probe_spp or min(config.spp, max(64, config.spp // 8)), sample_offset=0, flags=0)
+    probe = replace(config, spp=probe_spp or _probe_spp(gs, config), sample_offset=0, flags=0)
     keys = list(space)
     base = gs.get_tuning()
     results = []

@@ -159,6 +159,13 @@ class GpuScene:
             setattr(t, k, v)
         check(self.lib.sky_cuda_scene_set_tuning(self.handle, ctypes.byref(t)), self.lib)
 
+    def queue_spp(self, config: RenderConfig) -> int:
+        """Samples per pixel from which a render of `config` runs the stage queues; with fewer it
+        runs the ray loop (sky_cuda_queue_chains)."""
+        chains = ctypes.c_uint64(0)
+        check(self.lib.sky_cuda_queue_chains(self.handle, config.tracking, ctypes.byref(chains)), self.lib)
+        return -(-chains.value // (config.pixels * self.band_count))
+
     @staticmethod
     def _c_config(config: RenderConfig, count_events: bool):
         c = config.to_c()
