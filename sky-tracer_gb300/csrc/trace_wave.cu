@@ -35,11 +35,13 @@ __global__ void __launch_bounds__(256) wave_prepare_kernel(const DevJob* __restr
 // both kernels (ms, ray loop against queues):
 //   merged layers      one species: 3.1 M chains 0.63 / 0.65, 4.2 M 0.79 / 0.75: 24 per lane;
 //                      four: 4.0 M 1.47 / 1.60, 5.4 M 1.86 / 1.81: 34 per lane
-//   residual carry     131 k 0.52 / 0.68, 262 k 0.63 / 0.62, 524 k 0.82 / 0.70: 2 per lane
+//   residual carry     one species: 131 k 0.52 / 0.68, 262 k 0.63 / 0.62, 524 k 0.82 / 0.70: 2 per lane;
+//                      four (64x32, 41 bands): 0.32 M 0.95 / 1.08, 0.47 M 1.12 / 1.15, 0.62 M 1.28 / 1.29,
+//                      0.78 M 1.45 / 1.35: 5 per lane
 //   segment restart    0.67 M 1.25 / 1.34, 1.0 M 1.63 / 1.12: 5 per lane
 uint64_t wave_queue_chains(uint32_t tracking, uint32_t aerosol_species, int sms) {
     const uint64_t per_lane = tracking == SKY_TRACKING_SEGMENT_RESTART  ? 5u
-                              : tracking == SKY_TRACKING_RESIDUAL_CARRY ? 2u
+                              : tracking == SKY_TRACKING_RESIDUAL_CARRY ? (aerosol_species == 1u ? 2u : 5u)
                               : aerosol_species == 1u                   ? 24u
                                                                         : 34u;
     return per_lane * 1024u * uint64_t(sms);
