@@ -87,7 +87,7 @@ __device__ __forceinline__ uint32_t item_at(uint32_t i, uint32_t bands, uint32_t
 // Warp 0 of a block runs the derivative's recurrence of 32 items, warp 1 the
 // Riccati-Bessel functions'.
 __global__ void __launch_bounds__(64) mie_recurrences_kernel(const MieItem* __restrict__ items, uint32_t bands,
-                                                             uint32_t radii, double2* __restrict__ dscratch,
+                                                             uint32_t radii, double2* __restrict__ series,
                                                              double2* __restrict__ riccati) {
     const uint32_t place = blockIdx.x * 32u + (threadIdx.x & 31u);
     if (place >= bands * radii) return;
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(64) mie_recurrences_kernel(const MieItem* __re
     if (threadIdx.x < 32u) {
         // D_{n-1} = n/(mx) - 1/(D_n + n/(mx)), D_nmx = 0
         const Cd inv_mx = cd(1.0, 0.0) / (x * cd(it.m_re, it.m_im));
-        double2* D = dscratch + it.doff;
+        double2* D = series + it.off + i;
         Cd d = cd(0.0, 0.0);
         for (uint32_t n = it.dterms; n >= 1u; --n) {
             const Cd t = double(n) * inv_mx;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(64) mie_recurrences_kernel(const MieItem* __re
             if (n <= it.terms + 1u) D[n - 1u] = make_double2(d.re, d.im);
         }
     } else {
-        double2* R = riccati + it.aoff + i;  // terms + 1 of an item: psi_n, chi_n from n = 0
+        double2* R = riccati + it.off + i;  // terms + 1 of an item: psi_n, chi_n from n = 0
         double psi0 = cos(x), psi1 = sin(x), chi0 = -sin(x), chi1 = cos(x);
         R[0] = make_double2(psi1, chi1);
         for (uint32_t n = 1u; n <= it.terms; ++n) {
@@ -127,11 +127,18 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// A warp per item, lane l the terms l + 1, l + 33, ...
+// The coefficients of a term in the 16 bytes of its D_n.
+__device__ __forceinline__ double2 pack(float a, float b, float c, float d) {
+    return make_double2(__hiloint2double(__float_as_int(b), __float_as_int(a)),
+                        __hiloint2double(__float_as_int(d), __float_as_int(c)));
+}
+
+// A warp per item, lane l the terms l + 1, l + 33, ...  A lane reads D_n and writes the
+// term's coefficients over it (arrays of their own took half as much memory again).
 __global__ void __launch_bounds__(128) mie_coefficients_kernel(const MieItem* __restrict__ items, uint32_t bands,
-                                                               uint32_t radii, const double2* __restrict__ dscratch,
+                                                               uint32_t radii, double2* __restrict__ series,
                                                                const double2* __restrict__ riccati,
-                                                               float4* __restrict__ ab, double* __restrict__ q) {
+                                                               double* __restrict__ q) {
     const uint32_t place = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (place >= bands * radii) return;  // whole warps
     const uint32_t i = item_at(place, bands, radii);
@@ -139,9 +146,8 @@ __global__ void __launch_bounds__(128) mie_coefficients_kernel(const MieItem* __
     const double x = it.x;
     const Cd m = cd(it.m_re, it.m_im);
     const Cd inv_m = cd(1.0, 0.0) / m;
-    const double2* D = dscratch + it.doff;
-    const double2* R = riccati + it.aoff + i;
-    float4* out = ab + it.aoff;
+    double2* const D = series + it.off + i;
+    const double2* R = riccati + it.off + i;
     double qsca = 0.0, qext = 0.0, gsum = 0.0;
     Cd a_end = cd(0.0, 0.0), b_end = cd(0.0, 0.0);  // of the 32 terms before
     for (uint32_t n0 = 0u; n0 < it.terms; n0 += 32u) {
@@ -158,7 +164,7 @@ __global__ void __launch_bounds__(128) mie_coefficients_kernel(const MieItem* __
             an = (psi * ta - cd(psi1, 0.0)) / (ta * xi - xi1);
             bn = (psi * tb - cd(psi1, 0.0)) / (tb * xi - xi1);
             const double fn = (2.0 * rn + 1.0) / (rn * (rn + 1.0));
-            out[n - 1u] = make_float4(float(fn * an.re), float(fn * an.im), float(fn * bn.re), float(fn * bn.im));
+            D[n] = pack(float(fn * an.re), float(fn * an.im), float(fn * bn.re), float(fn * bn.im));
             qsca += (2.0 * rn + 1.0) * (norm2(an) + norm2(bn));
             qext += (2.0 * rn + 1.0) * (an.re + bn.re);
             gsum += fn * (an.re * bn.re + an.im * bn.im);
@@ -202,7 +208,7 @@ __device__ __forceinline__ void add_square(float& hi, float& lo, float v) {
 // Band blockIdx.x, radii blockIdx.y, + gridDim.y, ..., tiles of bins blockIdx.z, + gridDim.z, ...
 constexpr uint32_t kAngleThreads = 256, kAngleBins = 4;
 __global__ void __launch_bounds__(kAngleThreads) mie_angles_kernel(const MieItem* __restrict__ items, uint32_t radii,
-                                                                   const float4* __restrict__ ab, uint32_t bins,
+                                                                   const float4* __restrict__ series, uint32_t bins,
                                                                    double* __restrict__ phase_acc) {
     extern __shared__ float4 coef[];
     constexpr uint32_t kTile = kAngleThreads * kAngleBins;
@@ -220,7 +226,8 @@ __global__ void __launch_bounds__(kAngleThreads) mie_angles_kernel(const MieItem
             const MieItem it = items[size_t(blockIdx.x) * radii + r];
             const uint32_t N = it.terms;
             __syncthreads();
-            for (uint32_t n = threadIdx.x; n < N; n += blockDim.x) coef[n] = ab[it.aoff + n];
+            const float4* terms = series + it.off + size_t(blockIdx.x) * radii + r + 1u;  // of n = 1, 2, ...
+            for (uint32_t n = threadIdx.x; n < N; n += blockDim.x) coef[n] = terms[n];
             __syncthreads();
             const double scale = it.weight / (2.0 * it.k * it.k);  // w / (2 k^2)
             float pi0[kAngleBins], pi1[kAngleBins], s1r[kAngleBins], s1i[kAngleBins], s2r[kAngleBins], s2i[kAngleBins];
@@ -266,14 +273,14 @@ __global__ void __launch_bounds__(kAngleThreads) mie_angles_kernel(const MieItem
 }  // namespace
 
 cudaError_t launch_mie_bake(const MieItem* items, uint32_t bands, uint32_t radii, uint32_t max_terms,
-                            double2* dscratch, double2* riccati, float4* ab, double* q, uint32_t bins,
-                            double* phase_acc, uint32_t sms, cudaStream_t stream) {
+                            double2* series, double2* riccati, double* q, uint32_t bins, double* phase_acc,
+                            uint32_t sms, cudaStream_t stream) {
     const uint32_t count = bands * radii;
     if (count == 0) return cudaSuccess;
-    mie_recurrences_kernel<<<(count + 31u) / 32u, 64, 0, stream>>>(items, bands, radii, dscratch, riccati);
+    mie_recurrences_kernel<<<(count + 31u) / 32u, 64, 0, stream>>>(items, bands, radii, series, riccati);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    mie_coefficients_kernel<<<(count + 3u) / 4u, 128, 0, stream>>>(items, bands, radii, dscratch, riccati, ab, q);
+    mie_coefficients_kernel<<<(count + 3u) / 4u, 128, 0, stream>>>(items, bands, radii, series, riccati, q);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t smem = size_t(max_terms) * sizeof(float4);
     if ((e = allow_shared_memory(reinterpret_cast<const void*>(mie_angles_kernel), smem)) != cudaSuccess) return e;
@@ -281,7 +288,8 @@ cudaError_t launch_mie_bake(const MieItem* items, uint32_t bands, uint32_t radii
     const uint32_t tiles = uint32_t((uint64_t(bins) + kAngleThreads * kAngleBins - 1u) / (kAngleThreads * kAngleBins));
     const uint64_t each = uint64_t(bands) * tiles;
     const uint32_t shares = std::min(radii, std::max(1u, uint32_t((4u * sms + each - 1u) / each)));
-    mie_angles_kernel<<<dim3(bands, shares, std::min(tiles, 65535u)), kAngleThreads, smem, stream>>>(items, radii, ab, bins, phase_acc);
+    mie_angles_kernel<<<dim3(bands, shares, std::min(tiles, 65535u)), kAngleThreads, smem, stream>>>(
+        items, radii, reinterpret_cast<const float4*>(series), bins, phase_acc);
     return cudaGetLastError();
 }
 

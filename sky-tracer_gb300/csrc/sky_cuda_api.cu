@@ -1404,7 +1404,7 @@ extern "C" int sky_cuda_bake_mie_phase(const SkyMieDistribution* dist, const dou
     if (!(wsum > 0.0)) return set_error(SKY_ERR_INVALID_CONFIG, "the size distribution has no weight on its radii");
     const double two_pi = 2.0 * 3.14159265358979323846;
     std::vector<MieItem> items(size_t(band_count) * D.r_count);
-    uint64_t aoff = 0, doff = 0;
+    uint64_t terms = 0, wanted = 0;  // of all items, and of their downward recurrences with them
     uint32_t max_terms = 0;
     for (uint32_t b = 0; b < band_count; ++b) {
         const double lam = wavelength_um[b], mre = refr_re[b], mim = refr_im[b];
@@ -1426,34 +1426,34 @@ extern "C" int sky_cuda_bake_mie_phase(const SkyMieDistribution* dist, const dou
             it.terms = mie_terms(it.x);
             const double mx = it.x * std::sqrt(mre * mre + mim * mim);
             it.dterms = uint32_t(std::max(double(it.terms), mx)) + 16u;
-            it.aoff = aoff;
-            it.doff = doff;
+            it.off = terms;
             it._pad = 0;
-            aoff += it.terms;
-            doff += uint64_t(it.dterms) + 1u;
+            terms += it.terms;
+            wanted += it.terms + (uint64_t(it.dterms) + 1u);
             max_terms = std::max(max_terms, it.terms);
         }
     }
-    if (doff * sizeof(double2) + aoff * sizeof(float4) > (uint64_t(16) << 30))
+    // the bound of a derivative's whole recurrence and of the coefficients, 16 bytes each; the two
+    // arrays below, terms + 1 entries of each item, stay under it
+    if (wanted * sizeof(double2) > (uint64_t(16) << 30))
         return set_error(SKY_ERR_INVALID_CONFIG, "bake too large: more than 16 GB of series scratch");
     int device = 0, sms = 1;
     if (cudaGetDevice(&device) != cudaSuccess) return set_error(SKY_ERR_NO_DEVICE, "no usable CUDA device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     DeviceScratch mem;
     MieItem* d_items = nullptr;
-    double2 *d_scr = nullptr, *d_ric = nullptr;
-    float4* d_ab = nullptr;
+    double2 *d_series = nullptr, *d_ric = nullptr;
     double *d_q = nullptr, *d_acc = nullptr;
     cudaError_t e;
-    if ((e = mem.alloc(&d_items, items.size())) || (e = mem.alloc(&d_scr, doff)) ||
-        (e = mem.alloc(&d_ric, aoff + items.size())) || (e = mem.alloc(&d_ab, aoff)) ||
+    if ((e = mem.alloc(&d_items, items.size())) || (e = mem.alloc(&d_series, terms + items.size())) ||
+        (e = mem.alloc(&d_ric, terms + items.size())) ||
         (e = mem.alloc(&d_q, items.size() * 3)) || (e = mem.alloc(&d_acc, size_t(band_count) * phase_bins)))
         return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "Mie bake scratch allocation", e);
     clear_stale_error();
     if ((e = cudaMemcpy(d_items, items.data(), items.size() * sizeof(MieItem), cudaMemcpyHostToDevice)) ||
         (e = cudaMemset(d_acc, 0, size_t(band_count) * phase_bins * sizeof(double))))
         return cuda_fail(SKY_ERR_COPY, "Mie bake upload", e);
-    if ((e = launch_mie_bake(d_items, band_count, D.r_count, max_terms, d_scr, d_ric, d_ab, d_q, phase_bins, d_acc,
+    if ((e = launch_mie_bake(d_items, band_count, D.r_count, max_terms, d_series, d_ric, d_q, phase_bins, d_acc,
                              uint32_t(sms), nullptr)))
         return cuda_fail(SKY_ERR_LAUNCH, "Mie bake kernels", e);
     std::vector<double> q(items.size() * 3);
