@@ -1254,6 +1254,25 @@ struct DeviceScratch {  // frees what it allocated when the call returns
     }
 };
 
+// A combination's score from its sums and selected distances.
+void score_result(const ScoreState& S, SkyComboScore& r) {
+    r = SkyComboScore{};
+    r.finite = S.count;
+    if (S.count == 0) {
+        r.mean = r.rmse = r.p50 = r.p90 = r.p95 = r.p99 = r.max = r.score = std::nan("");
+        return;
+    }
+    r.mean = S.sum / double(S.count);
+    r.rmse = std::sqrt(S.sum_sq / double(S.count));
+    double* slot[kScoreTargets] = {&r.p50, &r.p90, &r.p95, &r.p99, &r.max};
+    for (uint32_t t = 0; t < kScoreTargets; ++t) {
+        float v;
+        std::memcpy(&v, &S.prefix[t], 4);
+        *slot[t] = double(v);
+    }
+    r.score = r.rmse + 0.25 * r.p95;
+}
+
 }  // namespace
 
 extern "C" int sky_cuda_score_reference(const double* ref_xyz, uint64_t samples, const double* scale_in,
@@ -1308,69 +1327,56 @@ extern "C" int sky_cuda_score_combos(const float* bands, uint32_t band_count, ui
         std::max<uint64_t>(1, std::min<uint64_t>({combo_count, 1024u, (uint64_t(1) << 24) / samples})));
     // whole groups of the distances' blocks (25 of 655 360 samples would leave the seventh three quarters empty)
     if (chunk < combo_count && chunk > kScoreGroup) chunk -= chunk % kScoreGroup;
-    // one allocation: the combinations, their states (all of them), one chunk's histograms and distances
+    // combinations whose states are held at a time (88 B each, their bands and weights)
+    const uint32_t pass = std::min(combo_count, 8192u);
+    // one allocation: a pass's combinations and their states, one chunk's histograms and distances
     size_t off = 0;
     auto reserve = [&off](size_t bytes) {
         const size_t at = off;
         off = align_up(off + bytes, 256);
         return at;
     };
-    const size_t o_state = reserve(size_t(combo_count) * sizeof(ScoreState));
+    const size_t o_state = reserve(size_t(pass) * sizeof(ScoreState));
     const size_t o_hist = reserve(size_t(chunk) * kScoreTargets * kScoreHistBins * sizeof(uint32_t));
     const size_t cleared = off;
-    const size_t o_bands = reserve(size_t(combo_count) * channels * sizeof(uint32_t));
-    const size_t o_xyz = reserve(size_t(combo_count) * channels * 3 * sizeof(float));
+    const size_t o_bands = reserve(size_t(pass) * channels * sizeof(uint32_t));
+    const size_t o_xyz = reserve(size_t(pass) * channels * 3 * sizeof(float));
     const size_t o_dist = reserve(size_t(chunk) * samples * sizeof(float));
     DeviceScratch mem;
     unsigned char* base = nullptr;
     cudaError_t e;
     if ((e = mem.alloc(&base, off))) return cuda_fail(SKY_ERR_OUT_OF_MEMORY, "scoring scratch allocation", e);
     clear_stale_error();
-    if ((e = cudaMemcpyAsync(base + o_bands, combo_bands, size_t(combo_count) * channels * sizeof(uint32_t),
-                             cudaMemcpyHostToDevice, stream)) ||
-        (e = cudaMemcpyAsync(base + o_xyz, combo_xyz, size_t(combo_count) * channels * 3 * sizeof(float),
-                             cudaMemcpyHostToDevice, stream)) ||
-        (e = cudaMemsetAsync(base, 0, cleared, stream)))
-        return cuda_fail(SKY_ERR_COPY, "scoring upload", e);
-    for (uint32_t c0 = 0; c0 < combo_count; c0 += chunk) {
-        ScoreLaunch w{};
-        w.bands = bands;
-        w.samples = samples;
-        w.ref_lab = ref_oklab;
-        w.inv_scale = 1.0f / reference_scale;
-        w.combo_bands = reinterpret_cast<const uint32_t*>(base + o_bands) + size_t(c0) * channels;
-        w.combo_xyz = reinterpret_cast<const float*>(base + o_xyz) + size_t(c0) * channels * 3;
-        w.combos = std::min(chunk, combo_count - c0);
-        w.channels = channels;
-        w.dist = reinterpret_cast<float*>(base + o_dist);
-        w.state = reinterpret_cast<ScoreState*>(base + o_state) + c0;
-        w.hist = reinterpret_cast<uint32_t*>(base + o_hist);
-        w.sms = uint32_t(sms);
-        if ((e = launch_score(w, stream))) return cuda_fail(SKY_ERR_LAUNCH, "scoring kernel launch", e);
-    }
-    std::vector<ScoreState> state(combo_count);
-    if ((e = cudaMemcpyAsync(state.data(), base + o_state, state.size() * sizeof(ScoreState), cudaMemcpyDeviceToHost,
-                             stream)) ||
-        (e = cudaStreamSynchronize(stream)))
-        return cuda_fail(SKY_ERR_SYNC, "scoring results", e);
-    for (uint32_t c = 0; c < combo_count; ++c) {
-        const ScoreState& S = state[c];
-        SkyComboScore& r = results[c];
-        r = SkyComboScore{};
-        r.finite = S.count;
-        if (S.count == 0) {
-            r.mean = r.rmse = r.p50 = r.p90 = r.p95 = r.p99 = r.max = r.score = std::nan("");
-            continue;
+    std::vector<ScoreState> state(pass);
+    for (uint64_t p0 = 0; p0 < combo_count; p0 += pass) {
+        const uint32_t n = uint32_t(std::min<uint64_t>(pass, combo_count - p0));
+        if ((e = cudaMemcpyAsync(base + o_bands, combo_bands + p0 * channels, size_t(n) * channels * sizeof(uint32_t),
+                                 cudaMemcpyHostToDevice, stream)) ||
+            (e = cudaMemcpyAsync(base + o_xyz, combo_xyz + p0 * channels * 3, size_t(n) * channels * 3 * sizeof(float),
+                                 cudaMemcpyHostToDevice, stream)) ||
+            (e = cudaMemsetAsync(base, 0, cleared, stream)))
+            return cuda_fail(SKY_ERR_COPY, "scoring upload", e);
+        for (uint32_t c0 = 0; c0 < n; c0 += chunk) {
+            ScoreLaunch w{};
+            w.bands = bands;
+            w.samples = samples;
+            w.ref_lab = ref_oklab;
+            w.inv_scale = 1.0f / reference_scale;
+            w.combo_bands = reinterpret_cast<const uint32_t*>(base + o_bands) + size_t(c0) * channels;
+            w.combo_xyz = reinterpret_cast<const float*>(base + o_xyz) + size_t(c0) * channels * 3;
+            w.combos = std::min(chunk, n - c0);
+            w.channels = channels;
+            w.dist = reinterpret_cast<float*>(base + o_dist);
+            w.state = reinterpret_cast<ScoreState*>(base + o_state) + c0;
+            w.hist = reinterpret_cast<uint32_t*>(base + o_hist);
+            w.sms = uint32_t(sms);
+            if ((e = launch_score(w, stream))) return cuda_fail(SKY_ERR_LAUNCH, "scoring kernel launch", e);
         }
-        r.mean = S.sum / double(S.count);
-        r.rmse = std::sqrt(S.sum_sq / double(S.count));
-        double* slot[kScoreTargets] = {&r.p50, &r.p90, &r.p95, &r.p99, &r.max};
-        for (uint32_t t = 0; t < kScoreTargets; ++t) {
-            float v;
-            std::memcpy(&v, &S.prefix[t], 4);
-            *slot[t] = double(v);
-        }
-        r.score = r.rmse + 0.25 * r.p95;
+        if ((e = cudaMemcpyAsync(state.data(), base + o_state, size_t(n) * sizeof(ScoreState), cudaMemcpyDeviceToHost,
+                                 stream)) ||
+            (e = cudaStreamSynchronize(stream)))
+            return cuda_fail(SKY_ERR_SYNC, "scoring results", e);
+        for (uint32_t c = 0; c < n; ++c) score_result(state[c], results[p0 + c]);
     }
     return SKY_OK;
 }
