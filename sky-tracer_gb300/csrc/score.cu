@@ -76,6 +76,11 @@ struct PairSum {
     }
 };
 
+// Bits of the distances from 2^-40 on and below 2^60, whose squares a PairSum holds: a
+// square's rounding error, a multiple of its exponent's 2^-46, is no denormal (those are
+// flushed to 0), and 32 squares' sum is finite.  The others' go to FP64.
+constexpr uint32_t kLeastSquare = (127u - 40u) << 23, kMostSquare = (127u + 60u) << 23;
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -140,14 +145,22 @@ __global__ void __launch_bounds__(256) distance_kernel(const float* __restrict__
                 xyz_to_oklab(x[j] * inv_scale, y[j] * inv_scale, z[j] * inv_scale, lab);
                 const float dl = lab[0] - l0[j], da = lab[1] - a0[j], db = lab[2] - b0[j];
                 float e = sqrtf(dl * dl + da * da + db * db);
-                if (!isfinite(e)) {
-                    e = __int_as_float(0x7fffffff);  // NaN: not counted, not selected
-                } else {
+                const uint32_t bits = __float_as_uint(e);
+                if (bits - kLeastSquare < kMostSquare - kLeastSquare) {
                     const float q = __fmul_rn(e, e);
                     s1[k].add(e, 0.0f);
                     s2[k].add(q, __fmaf_rn(e, e, -q));
                     ++n[k];
-                    atomicAdd(&h[k][__float_as_uint(e) >> 21], 1u);
+                    atomicAdd(&h[k][bits >> 21], 1u);
+                } else if (isfinite(e)) {
+                    if (e != 0.0f) {
+                        t1[k] += double(e);
+                        t2[k] += double(e) * double(e);
+                    }
+                    ++n[k];
+                    atomicAdd(&h[k][bits >> 21], 1u);
+                } else {
+                    e = __int_as_float(0x7fffffff);  // NaN: not counted, not selected
                 }
                 dist[size_t(c) * samples + at[j]] = e;
             }
