@@ -46,7 +46,10 @@ def score_combos(bands, ref_xyz: np.ndarray, combo_bands, combo_xyz, scale: floa
     bands = bands.contiguous()
     n = bands.shape[1]
     # the reference's scale and Oklab on the GPU (reference_scale() and oklab() in FP64)
-    ref = torch.as_tensor(np.ascontiguousarray(ref_xyz, dtype=np.float64).reshape(n, 3), device=bands.device)
+    ref = np.ascontiguousarray(ref_xyz, dtype=np.float64).reshape(n, 3)
+    if not ref.flags.writeable:
+        ref = ref.copy()  # torch warns of read-only arrays
+    ref = torch.as_tensor(ref, device=bands.device)
     ref_lab = torch.empty((n, 3), dtype=torch.float32, device=bands.device)
     st = torch.cuda.current_stream().cuda_stream if stream is None else stream
     used = ctypes.c_double(0.0)
