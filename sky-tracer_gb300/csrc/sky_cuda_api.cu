@@ -175,9 +175,9 @@ int validate_config(const SkyScene* scene, const SkyRenderConfig* c) {
         return set_error(SKY_ERR_INVALID_CONFIG, "row_begin needs a nonzero row_count");
     if (uint64_t(c->row_begin) + c->row_count > c->height)
         return set_error(SKY_ERR_INVALID_CONFIG, "rows [row_begin, row_begin + row_count) exceed the image height");
-    // the reference's own limit is on the whole image (integrator.rs:143-147)
-    uint64_t cells = uint64_t(c->width) * c->height * scene->dev.band_count;
-    if (cells > 0xffffffffull)
+    // the reference's own limit is on the whole image (integrator.rs:143-147); the pixels fit 64 bits,
+    // their product with the bands may not
+    if (uint64_t(c->width) * c->height > 0xffffffffull / scene->dev.band_count)
         return set_error(SKY_ERR_INVALID_CONFIG, "film is too large for the GPU shader index type");
     if (uint64_t(c->sample_offset) + c->spp > 0xffffffffull)
         return set_error(SKY_ERR_INVALID_CONFIG, "sample indices overflow 32 bits");
