@@ -268,7 +268,7 @@ typedef struct SkyTuning {
     uint32_t iteration_limit;    /* backstop of the wavefront kernel: loop iterations (one ray
                                     per lane each, or four batches of the stage queues) a warp
                                     may run before it stops and reports SKY_ERR_WATCHDOG;
-                                    0 = 2^31.  A render needs about 3 x chains / (32 x resident
+                                    0 = 2^31 (2^32 - 1 batches).  A render needs about 3 x chains / (32 x resident
                                     warps) iterations per warp.                              */
     uint32_t _reserved[2];
 } SkyTuning;

@@ -102,10 +102,9 @@ cudaError_t launch_adjoint_prepare(const AdjCtx& A, const AdjWorkspace& W, cudaS
 
 // Primal render over the parameterised medium: per-cell sums (and squares)
 // of the radiance of P, sampled with Q.  With P = Q it runs the ray loop of
-// the adjoint kernel (next_cell is its work counter); otherwise a warp per
-// cell.
-// A batch (J) takes the ray loop and needs P = Q; the warp-per-cell form
-// renders J.j[0] alone.
+// the adjoint kernel, or with enough chains and no counters the stage queues
+// (next_cell is their work counter); otherwise a warp per cell.
+// A batch (J) needs P = Q; the warp-per-cell form renders J.j[0] alone.
 cudaError_t launch_adjoint_primal(const AdjCtx& A, const AdjJobs& J, bool accumulate, unsigned long long* counters,
                                   uint32_t* status, unsigned long long* next_cell, cudaStream_t stream);
 

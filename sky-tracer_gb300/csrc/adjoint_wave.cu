@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 
     for (uint32_t batch = 0u;;) {
         uint32_t stage, take, id;
-        const Taken taken = queues.take(lane, turn, idle, batch, 0xffffffffu, status, stage, take, id);
+        const Taken taken = queues.take<wave::kMaxIdlePolls, false>(lane, turn, idle, batch, 0u, status, stage, take, id);
         if (taken == kOutOfWork) break;
         if (taken == kNothing) continue;
         if (kGrad && copies && batch % kFlushBatches == warp * (kFlushBatches / uint32_t(kWarps))) {

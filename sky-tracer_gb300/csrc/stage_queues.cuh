@@ -69,7 +69,8 @@ struct StageQueues {
     // The whole warp: up to 32 paths of one stage (lane i < take has path `id`).
     // `turn` is the stage that the warp prefers, `batch` counts its batches, `idle` its
     // polls of empty queues, under the low bits of the batch count that they came after.
-    template <uint32_t kMaxPolls = kMaxIdlePolls>
+    // `batch_limit`: batches before status bit 2 (kLimited).
+    template <uint32_t kMaxPolls = kMaxIdlePolls, bool kLimited = true>
     __device__ __forceinline__ Taken take(uint32_t lane, uint32_t& turn, uint32_t& idle, uint32_t& batch,
                                           uint32_t batch_limit, uint32_t* status, uint32_t& stage, uint32_t& count,
                                           uint32_t& id) const {
@@ -108,7 +109,7 @@ struct StageQueues {
             __syncwarp();
             return kNothing;
         }
-        if (batch >= batch_limit) {  // warp-uniform
+        if (kLimited && batch >= batch_limit) {  // warp-uniform
             if (lane == 0u) atomicOr(status, 2u);
             return kOutOfWork;
         }

@@ -56,7 +56,9 @@ namespace sky {
 namespace wave {
 
 // Batches of a warp that count as one iteration of SkyTuning.iteration_limit (32
-// chains take about 3.7 batches and 3 rays).
+// chains take about 3.7 batches and 3 rays).  The batches are counted in 32 bits: a
+// limit above 2^30 iterations, the default among them, is 2^32 - 1 batches, which take
+// as many chains as 2^31 iterations of the ray loop.
 constexpr uint64_t kBatchesPerIteration = 4;
 
 // Rays still under way when a warp leaves the tracking loop and puts them back:

@@ -2,7 +2,8 @@
 // path to each other: a warp holds it for some 30 us, puts it, and waits until
 // the other has taken it (at most 2 ms).  A warp's polls of empty queues end it
 // after kPolls in a row: far more than one wait takes, far fewer than all do.
-// Prints "<takes of warp 0> <takes of warp 1> <status>".
+// Prints "<takes of warp 0> <takes of warp 1> <status>", and of a warp that has had
+// 2^32 - 1 batches and takes another without a limit "<taken> <batches> <status>".
 
 #include <cstdio>
 
@@ -41,11 +42,25 @@ __global__ void __launch_bounds__(64) pass_a_path(uint32_t* out, uint32_t* statu
     if (lane == 0u) out[threadIdx.x >> 5] = batch;
 }
 
+__global__ void __launch_bounds__(32) one_more(uint32_t* out, uint32_t* status) {
+    __shared__ __align__(16) unsigned char smem[sizeof(Queues) + kQueues * 32u * sizeof(uint16_t)];
+    const StageQueues queues(reinterpret_cast<Queues*>(smem), 32u, 1u);
+    __syncthreads();
+    uint32_t turn = 0u, idle = 0u, batch = ~0u, stage = 0u, count = 0u, id = 0u;
+    const Taken taken =
+        queues.take<kMaxIdlePolls, false>(threadIdx.x, turn, idle, batch, 0u, status, stage, count, id);
+    if (threadIdx.x == 0u) {
+        out[0] = taken == kBatch;
+        out[1] = batch;
+    }
+}
+
 int main() {
-    uint32_t *d = nullptr, h[3] = {};
+    uint32_t *d = nullptr, h[6] = {};
     if (cudaMalloc(&d, sizeof(h)) != cudaSuccess || cudaMemset(d, 0, sizeof(h)) != cudaSuccess) return 1;
     pass_a_path<<<1, 64>>>(d, d + 2);
+    one_more<<<1, 32>>>(d + 3, d + 5);
     if (cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
-    std::printf("%u %u %u\n", h[0], h[1], h[2]);
+    std::printf("%u %u %u\n%u %u %u\n", h[0], h[1], h[2], h[3], h[4], h[5]);
     return 0;
 }

@@ -1,6 +1,6 @@
 """The stage queues' backstop counts a warp's polls of empty queues in a row, not
 over the whole launch: a launch of many minutes whose warps idle now and then
-runs on."""
+runs on.  Nor does a launch without a limit on its batches end at the 2^32-th."""
 
 import subprocess
 import sys
@@ -24,10 +24,19 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.gpu
-def test_a_batch_ends_the_count_of_empty_polls(gpu, harness):
+def _run(harness):
     res = subprocess.run([str(harness)], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stderr
-    first, second, status = map(int, res.stdout.split())
+    return [tuple(map(int, line.split())) for line in res.stdout.splitlines()]
+
+
+@pytest.mark.gpu
+def test_no_limit_on_the_batches(gpu, harness):
+    assert _run(harness)[1] == (1, 0, 0)  # the count starts again from 0
+
+
+@pytest.mark.gpu
+def test_a_batch_ends_the_count_of_empty_polls(gpu, harness):
+    first, second, status = _run(harness)[0]
     # 200 takes end the one, 199 or 200 the other
     assert status == 0 and max(first, second) == 200 and min(first, second) >= 199
