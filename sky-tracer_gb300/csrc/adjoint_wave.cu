@@ -17,11 +17,11 @@
 // What bounds it: instruction issue, as the tracer.  The ray loop runs all event
 // code once per ray: 8 to 10 of 32 lanes active.  16.8 M chains (128x64, 32 bands,
 // 64 spp): primal 3.79 -> 2.18 ms, gradient with the primal's chain radiance 4.05 ->
-// 3.00 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.1 ms and
+// 3.04 ms; 67 M chains (16 renders of 256x128, 4 bands, 32 spp): 19.4 -> 10.1 ms and
 // 29.7 -> 20.2 ms.  The primal issues at 83 % with 24 lanes active; the gradient at
-// 52 % with 17: its code is still more than the instruction caches hold ("no
-// instruction" 3.0 cycles per issue), and its layer gradients are shared-memory
-// atomics (short scoreboard 2.3, with one copy a warp).
+// 53 % with 17: its code is still more than the instruction caches hold ("no
+// instruction" 2.9 cycles per issue), and its layer gradients are shared-memory
+// atomics (short scoreboard 2.2).
 
 #include <algorithm>
 
@@ -174,7 +174,7 @@ __device__ __forceinline__ uint32_t adj_track_batch(const AdjCtx& A, bool alive,
 
 // The sums of the Rayleigh and Mie terms of a phase value or pdf with their
 // roundings written out, as the compiler contracts them in the ray loop: the two
-// kernels' chains then agree to the last bit but for one in a thousand.
+// kernels' chains then agree to the last bit but for two in a thousand.
 __device__ __forceinline__ float mixed(const AdjMed& m, float rayleigh, float mie) {
     const float r = __fmul_rn(m.R, rayleigh);
     return m.Ms > 0.0f ? __fmaf_rn(m.Ms, mie, r) : r;
